@@ -86,7 +86,7 @@ TRAFFIC_TABLE = os.path.join(ROOT, "profiles", "dram_traffic_rmat22.md")
 def kernel_name(kind, batched):
     return {"expand": "k_coop_fast" if batched else "k_expand_warp", "select": "k_select_fast",
             "select_thread": "k_select_thread",
-            "hub": "k_select_hub", "pair": "k_select_pair", "heavy": "k_expand_heavy",
+            "hub": "k_select_hub", "pair": "k_select_group", "heavy": "k_expand_heavy",
             "walk": "k_walk_fast" if batched else "k_walk_warp",
             "walk_thread": "k_walk_thread_fast" if batched else "k_walk_thread", "setup": "setup"}[kind]
 

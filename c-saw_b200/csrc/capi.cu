@@ -221,6 +221,10 @@ struct csaw_graph_s {
 
 namespace {
 
+// Prefix index levels begin on a 128-byte line (32 floats), as the lines the
+// searches probe do.
+int64_t line_align(int64_t n) { return (n + 31) & ~31ll; }
+
 // The plain schedule sees the per-edge degree array and the prefix cache only
 // when the caller asked for them at creation; the batched schedules
 // materialise them on first use.  `bias` selects the prefix cache (-1: none).
@@ -235,8 +239,8 @@ DevGraph dev_view(const csaw_graph_s *g, int schedule = CSAW_SCHED_BATCHED, int 
     d.ebias = (schedule != CSAW_SCHED_PLAIN || g->ebias_flag) ? g->ebias : nullptr;
     const bool fast = schedule != CSAW_SCHED_PLAIN;
     d.cdf = ((fast || g->cdf_flag) && bias > 0 && bias < 4) ? g->cdf[bias] : nullptr;
-    d.cdf1 = d.cdf ? d.cdf + g->E : nullptr;
-    d.cdf2 = d.cdf ? d.cdf + g->E + ((g->E + 31) >> 5) : nullptr;
+    d.cdf1 = d.cdf ? d.cdf + line_align(g->E) : nullptr;
+    d.cdf2 = d.cdf ? d.cdf1 + line_align((g->E + 31) >> 5) : nullptr;
     d.cdf_bias = bias;
     d.nrec = fast ? g->nrec : nullptr;
     d.tsc = (d.cdf && g->incr_rebuild) ? g->tsc[bias] : nullptr;
@@ -324,10 +328,9 @@ int ensure_cdf(csaw_graph_s *g, cudaStream_t st) {
     if (g->E == 0 || g->cdf_off) return 0;
     float *cdf = nullptr;   // prefix [E], then its search index levels [n1] and [n2]
     const int64_t n1 = (g->E + 31) >> 5, n2 = (g->E + 1023) >> 10;
+    const int64_t o1 = line_align(g->E), o2 = o1 + line_align(n1);
     ++g_alloc_epoch;
-    // + 16 floats: a row's 16-byte-aligned bulk-copy window may end up to 12
-    // bytes past the row (kernels_fast.cuh, k_select_pair)
-    CK(cudaMalloc((void **)&cdf, sizeof(float) * (size_t)(g->E + n1 + n2 + 16)));
+    CK(cudaMalloc((void **)&cdf, sizeof(float) * (size_t)(o2 + n2)));
     const DevGraph dg = dev_view(g);
     {
         LaunchScope ls(g, KK_INIT, st);
@@ -344,7 +347,7 @@ int ensure_cdf(csaw_graph_s *g, cudaStream_t st) {
     }
     {
         LaunchScope ls(g, KK_INIT, st);
-        k_cdf_index<<<g->sm_count * 4, 256, 0, st>>>(cdf, g->E, cdf + g->E, n1, cdf + g->E + n1, n2);
+        k_cdf_index<<<g->sm_count * 4, 256, 0, st>>>(cdf, g->E, cdf + o1, n1, cdf + o2, n2);
     }
     float2 *tsc = nullptr;   // tile summaries of the hub rows (incremental rebuilds)
     if (g->n_tsc > 0) {
@@ -359,7 +362,7 @@ int ensure_cdf(csaw_graph_s *g, cudaStream_t st) {
     CK(cudaStreamSynchronize(st));
     g->cdf[BIAS] = cdf;
     g->tsc[BIAS] = tsc;
-    g->dev_bytes += 4 * (g->E + n1 + n2);
+    g->dev_bytes += 4 * (g->E + n1 + n2);   // the levels themselves, without their padding
     ++g_alloc_epoch;
     return 0;
 }
@@ -528,7 +531,7 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
     const SchedArgs *sched = nullptr;
     const int hgrid = plain ? 0 : std::max(1, grid_for(k_select_hub<I, BIAS>, FAST_THREADS, 0, g->sm_count) *
                                                      g->grid_pct / 100);
-    const int pgrid = plain ? 0 : std::max(1, grid_for(k_select_pair<I, BIAS>, FAST_THREADS, 0, g->sm_count) *
+    const int pgrid = plain ? 0 : std::max(1, grid_for(k_select_group<I, BIAS>, FAST_THREADS, 0, g->sm_count) *
                                                      g->grid_pct / 100);
     if (BIASED && (!plain || g->cdf_flag)) TRY((ensure_cdf<I, BIAS>(g, st)));
     const bool cached = BIASED && g->cdf[BIAS] && (!plain || g->cdf_flag);
@@ -602,14 +605,8 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
     bool persist = !plain && g->persistent && !dedup && D <= PERSIST_MAX_LEVELS &&
                    (!sched || g->sched_host.mode == SCHED_THRESHOLD) && (!BIASED || cached);
     if (persist) {
-        static uint64_t attr_set = 0;   // per instantiation: bit = device
-        if (g->device < 64 && !((attr_set >> g->device) & 1u)) {
-            CK(cudaFuncSetAttribute(k_persist<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)PERSIST_SMEM));
-            attr_set |= 1ull << g->device;
-        }
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<I, BIAS>, FAST_THREADS, PERSIST_SMEM));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_persist<I, BIAS>, FAST_THREADS, 0));
         jgrid = per_sm * g->sm_count;   // all CTAs resident (cooperative launch)
         const bool retries = cached && g->maxdeg > WF;
         if (jgrid < 1 || (retries && (int64_t)jgrid * hstride * 4 > SCRATCH_BUDGET)) persist = false;
@@ -742,7 +739,6 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)jgrid);
             cfg.blockDim = dim3(FAST_THREADS);
-            cfg.dynamicSmemBytes = PERSIST_SMEM;
             cfg.stream = st;
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeCooperative;
@@ -808,7 +804,7 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
             if (a.pair_list) {
                 {
                     LaunchScope ls(g, KK_PAIR, st);
-                    k_select_pair<I, BIAS><<<pgrid, FAST_THREADS, 0, st>>>(dg, a);
+                    k_select_group<I, BIAS><<<pgrid, FAST_THREADS, 0, st>>>(dg, a);
                 }
                 LevelArgs ar = a;   // paired items that need a rebuild, redone by whole warps
                 ar.sel_list = a.refill_list;

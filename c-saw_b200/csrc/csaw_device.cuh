@@ -144,7 +144,7 @@ __device__ __forceinline__ int search_upper32(const float *P, int d, float t) {
 }
 
 // The same index by binary lifting in a fixed LOG steps, for d <= 2^LOG: no
-// data-dependent loop (lanes and half-warps searching rows of different
+// data-dependent loop (lanes searching rows of different
 // lengths stay converged); the last element is never read.
 template <int LOG>
 __device__ __forceinline__ int search_upper_lift(const float *P, int d, float t) {
@@ -195,22 +195,77 @@ __device__ __forceinline__ int64_t warp_search_upper(const float *P, int64_t d, 
     return lo + (__ffs(__ballot_sync(FULL, up)) - 1);
 }
 
-// First i in [0, d) with P[i] > t for the row of global edge offset beg of a
-// cached prefix, through its two index levels: a binary search of the
-// row's 1024-edge groups in cdf2 (E/1024 floats, L2-resident), then of the
-// group's 32-edge tiles in cdf1 and of the tile in cdf (each one 128-byte
-// line).  Every probe lies inside the row; the last candidate of each level
-// is known to exceed t (it ends the row, or ends the previous level's pick).
-__device__ __forceinline__ int64_t cdf_search(const DevGraph &g, int64_t beg, int64_t d, float t) {
-    const int64_t end = beg + d;
-    const int64_t ua = beg >> 10, ub = (end - 1) >> 10;
-    const int64_t u = ua + search_upper(g.cdf2 + ua, ub - ua + 1, t);
-    const int64_t ka = (u << 5) > (beg >> 5) ? (u << 5) : (beg >> 5);
-    const int64_t kb = (u << 5) + 31 < ((end - 1) >> 5) ? (u << 5) + 31 : ((end - 1) >> 5);
-    const int64_t k = ka + search_upper(g.cdf1 + ka, kb - ka + 1, t);
-    const int64_t ia = (k << 5) > beg ? (k << 5) : beg;
-    const int64_t ib = (k << 5) + 31 < end - 1 ? (k << 5) + 31 : end - 1;
-    return ia + search_upper(g.cdf + ia, ib - ia + 1, t) - beg;
+// First i in [lo, hi) with line[i] > t (line[hi - 1] > t is known and not
+// read) of a 32-entry line of a cached prefix or of its index: the last
+// entries of the line's first three 32-byte sectors are probed together, then
+// the sector found is searched (it is cached by then, but for the fourth).
+// Three loads in flight and three short ones after them, where a binary
+// search would wait for two or three sectors in turn.
+struct LineProbes {
+    float p0, p1, p2;
+};
+__device__ __forceinline__ LineProbes line_probes(const float *line, int lo, int hi) {
+    const float none = __int_as_float(0x7f800000);   // at or past the last entry: the answer lies before
+    const unsigned n = (unsigned)(hi - 1 - lo);
+    LineProbes r;
+    r.p0 = 7 < lo ? -none : none;
+    r.p1 = 15 < lo ? -none : none;
+    r.p2 = 23 < lo ? -none : none;
+    if ((unsigned)(7 - lo) < n) r.p0 = __ldg(line + 7);
+    if ((unsigned)(15 - lo) < n) r.p1 = __ldg(line + 15);
+    if ((unsigned)(23 - lo) < n) r.p2 = __ldg(line + 23);
+    return r;
+}
+__device__ __forceinline__ int line_find(const float *line, const LineProbes &r, int lo, int hi, float t) {
+    const int s = (r.p0 <= t ? 8 : 0) + (r.p1 <= t ? 8 : 0) + (r.p2 <= t ? 8 : 0);
+    int at = s > lo ? s : lo;
+    const int end = s + 7 < hi - 1 ? s + 7 : hi - 1;
+#pragma unroll
+    for (int step = 4; step >= 1; step >>= 1) {
+        const int i = at + step - 1;
+        if (i < end && !(__ldg(line + i) > t)) at += step;
+    }
+    return at;
+}
+
+// First i in [0, d) with P[i] > its_target(x, T) for the row [beg, beg + d) of
+// a cached prefix, through its two index levels: the row's 1024-edge groups
+// in cdf2 (E/1024 floats, L2-resident), the group's 32-edge tiles in cdf1,
+// the tile in cdf (each of these one line).  Every probe lies inside the row;
+// the last candidate of each level is known to exceed the target (it ends the
+// row, or ends the previous level's pick).  Positions are relative to the row
+// in 32 bits, and only rows of several groups loop, so lanes on different
+// rows stay converged; the first tile line's probes do not wait for T.
+__device__ __forceinline__ int cdf_find(const DevGraph &g, int64_t beg, int d, uint32_t x, float T) {
+    const int o1 = (int)(beg & 31), o2 = (int)(beg & 1023);   // the row's start in its tile and group
+    const int last = d - 1;
+    const float *c1 = g.cdf1 + ((beg >> 10) << 5);            // the tiles of the row's first group
+    const int kend = (int)(((unsigned)o2 + (unsigned)last) >> 5);                        // its last tile, from there
+    int lo = o2 >> 5, hi = kend < 31 ? kend + 1 : 32;
+    LineProbes r = line_probes(c1, lo, hi);
+    const float t = its_target(x, T);
+    int top = (int)(((unsigned)o2 + (unsigned)last) >> 10);
+    if (top > 0) {
+        const float *c2 = g.cdf2 + (beg >> 10);
+        int u = 0;
+#pragma unroll 1
+        while (u < top) {
+            const int mid = (u + top) >> 1;
+            if (__ldg(c2 + mid) > t) top = mid; else u = mid + 1;
+        }
+        if (u > 0) {
+            c1 += u << 5;
+            lo = 0;
+            hi = kend - (u << 5) < 31 ? kend - (u << 5) + 1 : 32;
+            r = line_probes(c1, lo, hi);
+        }
+        top = u;
+    }
+    const int k = (top << 5) + line_find(c1, r, lo, hi, t) - (o2 >> 5);   // the tile, from the row's first
+    const float *line = g.cdf + (beg - o1) + (k << 5);
+    const int e0 = (k << 5) - o1;                                          // its first edge, from the row's
+    const int a = e0 < 0 ? -e0 : 0, b = last - e0 < 31 ? last - e0 + 1 : 32;
+    return e0 + line_find(line, line_probes(line, a, b), a, b, t);
 }
 
 // The same with one warp-uniform target, each level by warp_search_upper.
@@ -245,9 +300,73 @@ __device__ __forceinline__ float warp_max_scan(float v, int lane) {
     return v;
 }
 
+// Passes of warp_canon_prefix over B tiles at once, tiles [t0, t0 + B) of
+// which the first `have` exist: the B shuffle chains are independent, so
+// their latencies (and the B bias loads) overlap.
+template <int B, typename WFn>
+__device__ __forceinline__ void canon_tiles_scan(WFn wfn, int64_t d, float *P, const uint32_t *zmask, int64_t t0,
+                                                 int have, int slot, float &my_tsum, int lane) {
+    float v[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int64_t i = ((t0 + u) << 5) + lane;
+        v[u] = u < have && i < d ? wfn(i) : 0.f;
+    }
+    if (zmask) {
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (u < have && ((zmask[t0 + u] >> lane) & 1u)) v[u] = 0.f;
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const float up = __shfl_up_sync(FULL, v[u], off);
+            if (lane >= off) v[u] = __fadd_rn(v[u], up);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int64_t i = ((t0 + u) << 5) + lane;
+        if (u < have && i < d) P[i] = v[u];
+        const float s = __shfl_sync(FULL, v[u], 31);
+        if (lane == slot + u) my_tsum = s;
+    }
+}
+
+template <int B>
+__device__ __forceinline__ void canon_tiles_finish(int64_t d, float *P, int64_t t0, int have, int slot, float C,
+                                                   float qex, float &runmax, int lane) {
+    float p[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int64_t i = ((t0 + u) << 5) + lane;
+        const float qx = __shfl_sync(FULL, qex, (slot + u) & 31);
+        p[u] = u < have && i < d ? __fadd_rn(C, __fadd_rn(qx, P[i])) : 0.f;
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            const float up = __shfl_up_sync(FULL, p[u], off);
+            if (lane >= off) p[u] = fmaxf(p[u], up);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+        const int64_t i = ((t0 + u) << 5) + lane;
+        p[u] = fmaxf(p[u], runmax);
+        if (u < have && i < d) P[i] = p[u];
+        if (u < have) runmax = __shfl_sync(FULL, p[u], 31);
+    }
+}
+
 // Canonical prefix of wfn(0..d) into P[0..d) computed by one warp; elements
 // whose bit is set in zmask (if given) count as 0.  Returns T = P[d-1] on
-// every lane.  P may live in shared or global memory.
+// every lane.  P may live in shared or global memory.  Four tiles at a time
+// (two where at most two are left): one tile after the other is a chain of
+// ten dependent shuffles and a load per tile, which made a rebuild of a
+// 512-edge row the longest part of a warp's item.
 template <typename WFn>
 __device__ float warp_canon_prefix(WFn wfn, int64_t d, float *P, const uint32_t *zmask, int lane) {
     const int64_t ntiles = (d + 31) >> 5;
@@ -255,31 +374,18 @@ __device__ float warp_canon_prefix(WFn wfn, int64_t d, float *P, const uint32_t 
     for (int64_t g0 = 0; g0 < ntiles; g0 += 32) {
         const int gt = (ntiles - g0) < 32 ? (int)(ntiles - g0) : 32;
         float my_tsum = 0.f;
-        for (int tt = 0; tt < gt; ++tt) {
-            int64_t i = ((g0 + tt) << 5) + lane;
-            float w = 0.f;
-            if (i < d) {
-                w = wfn(i);
-                if (zmask && ((zmask[i >> 5] >> (i & 31)) & 1u)) w = 0.f;
-            }
-            float v = warp_ks_sum(w, lane);
-            if (i < d) P[i] = v;
-            float s = __shfl_sync(FULL, v, 31);
-            if (lane == tt) my_tsum = s;
+        for (int tt = 0; tt < gt; tt += 4) {
+            if (gt - tt <= 2) canon_tiles_scan<2>(wfn, d, P, zmask, g0 + tt, gt - tt, tt, my_tsum, lane);
+            else canon_tiles_scan<4>(wfn, d, P, zmask, g0 + tt, gt - tt, tt, my_tsum, lane);
         }
-        float q = warp_ks_sum(my_tsum, lane);
+        const float q = warp_ks_sum(my_tsum, lane);
         float qex = __shfl_up_sync(FULL, q, 1);
         if (lane == 0) qex = 0.f;
-        float gtot = __shfl_sync(FULL, q, 31);
+        const float gtot = __shfl_sync(FULL, q, 31);
         __syncwarp();
-        for (int tt = 0; tt < gt; ++tt) {
-            int64_t i = ((g0 + tt) << 5) + lane;
-            float qx = __shfl_sync(FULL, qex, tt);
-            float p = 0.f;
-            if (i < d) p = __fadd_rn(C, __fadd_rn(qx, P[i]));
-            p = fmaxf(warp_max_scan(p, lane), runmax);
-            if (i < d) P[i] = p;
-            runmax = __shfl_sync(FULL, p, 31);
+        for (int tt = 0; tt < gt; tt += 4) {
+            if (gt - tt <= 2) canon_tiles_finish<2>(d, P, g0 + tt, gt - tt, tt, C, qex, runmax, lane);
+            else canon_tiles_finish<4>(d, P, g0 + tt, gt - tt, tt, C, qex, runmax, lane);
         }
         C = __fadd_rn(C, gtot);
     }
@@ -403,10 +509,10 @@ struct SlotRng {
 };
 
 // Resolver state of the warp-parallel sequential-order selection: lane j owns
-// slot j.  j (current slot) and a (draws in this phase for slot j) are warp
-// uniform; A (draws used by the lane's slot), cand and sel are per lane.
+// slot j.  j (current slot) is warp uniform; A (draws used by the lane's
+// slot), a (those of this phase), cand and sel are per lane.
 struct SelState {
-    int j = 0, a = 1, A = 0;
+    int j = 0, A = 0, a = 1;
     int cand = -1, sel = -1;
 };
 
@@ -416,44 +522,41 @@ struct SelState {
 // has exhausted its REJECT_ATTEMPTS draws in this phase (returns 1: rebuild).
 // A slot that has used MAX_SLOT_DRAWS draws takes the smallest unselected
 // index, so the loop always ends.
+// A round accepts the run of slots whose candidates repeat no lower slot's,
+// up to the first slot f that repeats one, and then draws again for every
+// slot whose candidate repeats an accepted selection: slot order would
+// reject exactly those draws when their turns come (draws are keyed by slot
+// and number), so slots that collide with the same heavy neighbor redraw in
+// one round instead of a round each.
 template <typename CandFn>
 __device__ __forceinline__ int resolve_slots(SelState &st, int N, int lane, const DrawCtx &dc,
                                              SlotRng &rng, CandFn cand_of) {
     while (st.j < N) {
-        // Accept in one step the run of slots j, j+1, ... whose current
-        // candidates repeat no lower slot's value (lanes below j hold their
-        // selections); the sequential order would accept each in turn.
         const int j0 = st.j;
         const int v = lane < j0 ? st.sel : (lane < N ? st.cand : -2 - lane);
-        const unsigned same = __match_any_sync(FULL, v);
-        const bool dup = lane >= j0 && lane < N && (same & ((1u << lane) - 1u)) != 0u;
+        const unsigned lower = __match_any_sync(FULL, v) & ((1u << lane) - 1u);
+        const bool dup = lane >= j0 && lane < N && lower != 0u;
         const unsigned db = __ballot_sync(FULL, dup);
-        const int j = db ? __ffs(db) - 1 : N;
-        if (lane >= j0 && lane < j) st.sel = v;
-        if (j == N) {
-            st.j = N;
-            st.a = 1;
-            return 0;
-        }
-        if (j > j0) st.a = 1;   // slot j rejects its first draw of this phase
-        st.j = j;
-        if (__shfl_sync(FULL, st.A, j) == MAX_SLOT_DRAWS) {
+        const int f = db ? __ffs(db) - 1 : N;
+        if (lane >= j0 && lane < f) st.sel = v;
+        st.j = f;
+        if (f == N) return 0;
+        if (__shfl_sync(FULL, st.A, f) == MAX_SLOT_DRAWS) {
             int i = 0;
-            while (__ballot_sync(FULL, lane < j && st.sel == i)) ++i;
-            if (lane == j) st.sel = i;
-            st.j = j + 1;
-            st.a = 1;
+            while (__ballot_sync(FULL, lane < f && st.sel == i)) ++i;
+            if (lane == f) st.sel = i;
+            st.j = f + 1;
             continue;
         }
-        if (st.a == REJECT_ATTEMPTS) return 1;
-        const bool me = lane == j;
-        const uint32_t x = me ? rng.word(dc, lane, st.A) : 0u;
-        const int nc = cand_of(x, me);  // warp-uniform call (may shuffle)
-        if (me) {
+        const bool again = dup && (lower & ((1u << f) - 1u)) != 0u && st.a < REJECT_ATTEMPTS;
+        if (!((__ballot_sync(FULL, again) >> f) & 1u)) return 1;   // slot f's draws of this phase ran out
+        const uint32_t x = again ? rng.word(dc, lane, st.A) : 0u;
+        const int nc = cand_of(x, again);  // warp-uniform call (may shuffle)
+        if (again) {
             st.cand = nc;
             st.A++;
+            st.a++;
         }
-        st.a++;
     }
     return 0;
 }

@@ -19,18 +19,20 @@
 //   - batch size shrinks on small levels so every warp gets work.
 #pragma once
 
-#include "bulk_copy.cuh"
 #include "kernels_sample.cuh"
 
 namespace csaw {
 
 constexpr int WF = 512;  // per-warp shared prefix capacity of the fast kernels
-// Resident CTAs per SM the pair kernel is compiled for (register budget).
-#ifndef CSAW_PAIR_MIN_BLOCKS
-#define CSAW_PAIR_MIN_BLOCKS 4
+// Resident CTAs per SM the group kernel is compiled for (register budget).
+#ifndef CSAW_GROUP_MIN_BLOCKS
+#define CSAW_GROUP_MIN_BLOCKS 6
 #endif
-// Cached items with N <= 16 and d >= this many times N go to the pair pass
-// (3: a phase-1 rejection is rare enough that its refill stays cheap).
+// Cached items with N <= 16 and d >= this many times N go to the group pass
+// (3: a phase-1 rejection is rare enough that its refill stays cheap; N =
+// 17..32, one item a warp, measured slower on the power-law batch, N = 20:
+// 0.26 -> 0.34 ms, as few rows are that long and each level pays for the
+// pass's launches).
 #ifndef CSAW_PAIR_MIN_RATIO
 #define CSAW_PAIR_MIN_RATIO 3
 #endif
@@ -124,36 +126,34 @@ __device__ __forceinline__ void preload_bias(const DevGraph &g, int64_t beg, int
 // A rejection phase allows REJECT_ATTEMPTS = 4 draws per slot, and the four
 // words of one Philox block are exactly the next four draws of a slot, so
 // every pending lane computes the candidates of its next four draws at once
-// (four independent searches, overlapped) and a rejected draw costs one
-// shuffle and one ballot instead of a serial search.
+// (four independent searches, overlapped) and a round of rejections costs a
+// match and two ballots instead of a search.
 struct Spec4 {
-    int j = 0, a = 1;   // warp uniform: current slot, draws it used in this window
+    int j = 0;          // warp uniform: current slot
+    int a = 1;          // lane: draws its slot has used in this window (cand is draw a - 1)
     int have = 4;       // warp uniform: candidates computed ahead per lane (4, or 1 when lazy)
-    int base = 0;       // lane: draw index of c0 (a multiple of 4)
-    int sel = -1;
-    int c0 = -1, c1 = -1, c2 = -1, c3 = -1;
-    __device__ __forceinline__ int pick(int k) const { return k == 0 ? c0 : (k == 1 ? c1 : (k == 2 ? c2 : c3)); }
+    int base = 0;       // lane: draw index of the window's first draw (a multiple of 4)
+    int sel = -1, cand = -1;
+    int c1 = -1, c2 = -1, c3 = -1;
 };
 
 // Windows of lanes [from, N): lane `from` starts at draw from_base, later
 // lanes at draw 0, all on the current prefix.  Warp-uniform.
 // lazy: compute only the first candidate of each window; later ones are
-// computed on demand for the rejected slot (for costly searches where a
-// rejection is rare, e.g. d >= 4N).
+// computed on demand for the rejected slots (where rejections are rare, e.g.
+// d >= 4N).
 template <typename CandFn>
 __device__ __forceinline__ void spec_fill(Spec4 &st, int from, int N, int lane, const DrawCtx &dc, SlotRng &rng,
                                           CandFn cand_of, int from_base, bool lazy) {
     const bool act = lane >= from && lane < N;
     const int base = lane == from ? from_base : 0;
+    st.a = 1;
+    if (act) st.base = base;
     if (lazy) {
         const uint32_t x0 = act ? rng.word(dc, lane, base) : 0u;
         const int n0 = cand_of(x0, act);
-        if (act) {
-            st.base = base;
-            st.c0 = n0;
-        }
+        if (act) st.cand = n0;
         st.have = 1;
-        st.a = 1;
         return;
     }
     uint32_t x0 = 0, x1 = 0, x2 = 0, x3 = 0;
@@ -165,14 +165,12 @@ __device__ __forceinline__ void spec_fill(Spec4 &st, int from, int N, int lane, 
     }
     const int n0 = cand_of(x0, act), n1 = cand_of(x1, act), n2 = cand_of(x2, act), n3 = cand_of(x3, act);
     if (act) {
-        st.base = base;
-        st.c0 = n0;
+        st.cand = n0;
         st.c1 = n1;
         st.c2 = n2;
         st.c3 = n3;
     }
     st.have = 4;
-    st.a = 1;
 }
 
 __device__ __forceinline__ void fill_smallest(Spec4 &st, int j, int lane) {
@@ -181,46 +179,36 @@ __device__ __forceinline__ void fill_smallest(Spec4 &st, int j, int lane) {
     if (lane == j) st.sel = i;
 }
 
-// 0: all N slots accepted; 1: slot st.j needs a phase rebuild.
+// 0: all N slots accepted; 1: slot st.j needs a phase rebuild.  Rounds as in
+// resolve_slots: every slot whose candidate repeats an accepted selection
+// goes on to its next draw in the same round.
 template <typename CandFn>
 __device__ __forceinline__ int resolve4(Spec4 &st, int N, int lane, const DrawCtx &dc, SlotRng &rng, CandFn cand_of) {
     while (st.j < N) {
-        const int j = st.j, a = st.a;
-        int cj;
-        if (a - 1 < st.have) {
-            cj = st.pick(a - 1);
-        } else {   // lazy window: the rejected slot's next draw, on its lane
-            const bool me = lane == j;
-            cj = cand_of(me ? rng.word(dc, lane, st.base + a - 1) : 0u, me);
-        }
-        // Accept in one step the run of slots j, j+1, ... whose current
-        // candidates repeat no lower slot's value: lanes below j hold their
-        // selections, lane j its draw a, lanes above their first draw (the
-        // sequential order would accept each of them in turn).  f is the first
-        // slot whose candidate repeats a lower one.
-        const int v = lane < j ? st.sel : (lane == j ? cj : (lane < N ? st.c0 : -2 - lane));
-        const unsigned same = __match_any_sync(FULL, v);
-        const bool dup = lane >= j && lane < N && (same & ((1u << lane) - 1u)) != 0u;
+        const int j0 = st.j;
+        const int v = lane < j0 ? st.sel : (lane < N ? st.cand : -2 - lane);
+        const unsigned lower = __match_any_sync(FULL, v) & ((1u << lane) - 1u);
+        const bool dup = lane >= j0 && lane < N && lower != 0u;
         const unsigned db = __ballot_sync(FULL, dup);
         const int f = db ? __ffs(db) - 1 : N;
-        if (lane >= j && lane < f) st.sel = v;
-        if (f == N) {
-            st.j = N;
-            st.a = 1;
-            return 0;
-        }
-        // slot f's current draw (draw a of slot j, or the first of a later slot) is rejected
-        const int af = f == j ? a : 1;
+        if (lane >= j0 && lane < f) st.sel = v;
         st.j = f;
-        if (__shfl_sync(FULL, st.base, f) + af == MAX_SLOT_DRAWS) {
+        if (f == N) return 0;
+        if (__shfl_sync(FULL, st.base + st.a, f) == MAX_SLOT_DRAWS) {
             fill_smallest(st, f, lane);
             st.j = f + 1;
-            st.a = 1;
             continue;
         }
-        st.a = af;
-        if (af == REJECT_ATTEMPTS) return 1;
-        st.a = af + 1;
+        const bool again = dup && (lower & ((1u << f) - 1u)) != 0u && st.a < REJECT_ATTEMPTS;
+        if (!((__ballot_sync(FULL, again) >> f) & 1u)) return 1;   // slot f's window ran out
+        if (st.have == 4) {
+            if (again) st.cand = st.a == 1 ? st.c1 : (st.a == 2 ? st.c2 : st.c3);
+        } else {   // lazy windows: the next draws of the rejected slots
+            const uint32_t x = again ? rng.word(dc, lane, st.base + st.a) : 0u;
+            const int nc = cand_of(x, again);
+            if (again) st.cand = nc;
+        }
+        if (again) st.a++;
     }
     return 0;
 }
@@ -238,27 +226,21 @@ __device__ __forceinline__ int select_spec(int N, int lane, const DrawCtx &dc, b
                                            RebuildFn rebuild, bool lazy = false, int j0 = 0, int sel0 = -1) {
     SlotRng rng;
     Spec4 st;
-    if (j0 > 0) {
-        st.j = j0;
-        st.sel = lane < j0 ? sel0 : -1;
-        if (!rebuild(st, j0)) zero = true;
-        else spec_fill(st, j0, N, lane, dc, rng, cand_of, REJECT_ATTEMPTS, lazy);
-    } else if (!zero) {
-        spec_fill(st, 0, N, lane, dc, rng, cand_of, 0, lazy);
-    }
+    bool again = j0 > 0;   // a phase failed: rebuild without the selections so far
+    int from = again ? j0 : 0, base = again ? REJECT_ATTEMPTS : 0;
+    if (again) st.sel = lane < j0 ? sel0 : -1;
+    st.j = from;
     for (;;) {
+        if (again && !rebuild(st, from)) zero = true;
         if (zero) {
-            for (int jj = st.j; jj < N; ++jj) fill_smallest(st, jj, lane);
+            for (int jj = from; jj < N; ++jj) fill_smallest(st, jj, lane);
             break;
         }
+        spec_fill(st, from, N, lane, dc, rng, cand_of, base, lazy);
         if (resolve4(st, N, lane, dc, rng, cand_of) == 0) break;
-        const int j = st.j;
-        const int next = __shfl_sync(FULL, st.base, j) + REJECT_ATTEMPTS;
-        if (!rebuild(st, j)) {
-            zero = true;
-            continue;
-        }
-        spec_fill(st, j, N, lane, dc, rng, cand_of, next, lazy);
+        from = st.j;
+        base = __shfl_sync(FULL, st.base, from) + REJECT_ATTEMPTS;
+        again = true;
     }
     return st.sel;
 }
@@ -490,7 +472,7 @@ __device__ __forceinline__ void coop_body(const DevGraph &g, const LevelArgs &a)
         // thread class: one item per thread (valid only with a thread list)
         const bool thr = drawn && cls == CLS_THREAD;
         const bool heavy = drawn && cls >= 2 && !thr;
-        // cached items with few slots and a rare rebuild run two per warp;
+        // cached items with few slots and a rare rebuild run 32 / N per warp;
         // other warp-class items above WF search the cached prefix in their own list
         const bool pair = drawn && !heavy && !thr && cached && N <= 16 && d >= CSAW_PAIR_MIN_RATIO * N && a.pair_list;
         const bool hub = drawn && !heavy && !thr && cached && d > WF && !pair;
@@ -807,264 +789,143 @@ k_select_thread(DevGraph g, LevelArgs a) {
     select_thread_body<I, BIAS>(g, a);
 }
 
-// Half-warp primitives: a warp runs two independent items, lanes 0-15 and
-// 16-31, each with its own mask (the halves may diverge).
-struct Half {
-    unsigned mask;
-    int base, sl;   // first lane of the half, lane within the half
-    __device__ explicit Half(int lane) : mask(0xFFFFu << (lane & 16)), base(lane & 16), sl(lane & 15) {}
-    __device__ int shfl(int v, int src) const { return __shfl_sync(mask, v, base + src); }
-    __device__ unsigned ballot(bool p) const { return (__ballot_sync(mask, p) >> base) & 0xFFFFu; }
-    __device__ unsigned match(int v) const { return (__match_any_sync(mask, v) >> base) & 0xFFFFu; }
-};
-
-// Draws of one item (N <= 16 slots) in a half-warp, slot j on lane j, the
-// same draws and acceptance order as resolve_slots; cand_of(x) is a per-lane
-// search.  Returns -1 when every slot is accepted, else the slot j whose
-// draws of the first phase ran out (slots below j then hold their accepted
-// indices in sel; the item needs a rebuild of its prefix, which a whole warp
-// or CTA goes on with).  T <= 0: the slots take indices 0..N-1.
-template <typename CandFn>
-__device__ __forceinline__ int half_select(const Half &h, int N, const DrawCtx &dc, float T, CandFn cand_of,
-                                           int &sel) {
-    const int sl = h.sl;
-    sel = sl;
-    if (!(T > 0.f)) return -1;
-    SlotRng rng;
-    int cand = -1, A = 0;
-    if (sl < N) {
-        cand = cand_of(rng.word(dc, sl, 0));
-        A = 1;
-    }
-    int j = 0, a = 1;
-    while (j < N) {
-        const int v = sl < j ? sel : (sl < N ? cand : -2 - sl);
-        const unsigned same = h.match(v);
-        const bool dup = sl >= j && sl < N && (same & ((1u << sl) - 1u)) != 0u;
-        const unsigned db = h.ballot(dup);
-        const int f = db ? __ffs(db) - 1 : N;
-        if (sl >= j && sl < f) sel = v;
-        if (f == N) break;
-        if (f > j) a = 1;
-        j = f;
-        if (h.shfl(A, j) == MAX_SLOT_DRAWS) {   // termination guard: smallest unselected index
-            int i = 0;
-            while (h.ballot(sl < j && sel == i)) ++i;
-            if (sl == j) sel = i;
-            ++j;
-            a = 1;
-            continue;
-        }
-        if (a == REJECT_ATTEMPTS) return j;
-        if (sl == j) {
-            cand = cand_of(rng.word(dc, sl, A));
-            ++A;
-        }
-        ++a;
-    }
-    return -1;
-}
-
-// What the pair kernel stages in shared memory for an item over a cached
-// prefix: its whole prefix row (d <= WF), else the row's entries of the
-// first prefix index level (cdf1, one per 32 edges) when they fit in WF
-// floats, else those of the second level (cdf2, one per 1024 edges), else
-// nothing (rows above ~512 K edges search the global index).
-enum : int { STAGE_NONE = 0, STAGE_ROW = 1, STAGE_CDF1 = 2, STAGE_CDF2 = 3 };
-struct StagePlan {
-    int mode;
-    const float *src;
-    int count;
-};
-
-__device__ __forceinline__ StagePlan stage_plan(const DevGraph &g, int64_t beg, int d) {
-    const int64_t end = beg + d;
-    if (d <= WF) return StagePlan{STAGE_ROW, g.cdf + beg, d};
-    const int64_t ka = beg >> 5, kb = (end - 1) >> 5;
-    if (kb - ka + 1 <= WF) return StagePlan{STAGE_CDF1, g.cdf1 + ka, (int)(kb - ka + 1)};
-    const int64_t ua = beg >> 10, ub = (end - 1) >> 10;
-    if (ub - ua + 1 <= WF) return StagePlan{STAGE_CDF2, g.cdf2 + ua, (int)(ub - ua + 1)};
-    return StagePlan{STAGE_NONE, nullptr, 0};
-}
-
-// cdf_search for an item whose index level is staged (STAGE_CDF1 /
-// STAGE_CDF2), once the staged entries' search has given r: the remaining
-// levels in global memory, one 32-entry line each, by fixed-step lifting.
-// The same index as cdf_search (the first i with P[i] > t is unique); as
-// there, no level reads its last candidate.
-__device__ __forceinline__ int64_t staged_refine(const DevGraph &g, int mode, int r, int64_t beg, int64_t d, float t) {
-    const int64_t end = beg + d;
-    int64_t k;
-    if (mode == STAGE_CDF1) {
-        k = (beg >> 5) + r;
-    } else {
-        const int64_t u = (beg >> 10) + r;
-        const int64_t ka = (u << 5) > (beg >> 5) ? (u << 5) : (beg >> 5);
-        const int64_t kb = (u << 5) + 31 < ((end - 1) >> 5) ? (u << 5) + 31 : ((end - 1) >> 5);
-        k = ka + search_upper_lift<5>(g.cdf1 + ka, (int)(kb - ka + 1), t);
-    }
-    const int64_t ia = (k << 5) > beg ? (k << 5) : beg;
-    const int64_t ib = (k << 5) + 31 < end - 1 ? (k << 5) + 31 : end - 1;
-    return ia + search_upper_lift<5>(g.cdf + ia, (int)(ib - ia + 1), t) - beg;
-}
-
-// Shared-memory copy of a work entry (three 16-byte loads).
-__device__ __forceinline__ SelEntry load_sel_smem(const SelEntry *e) {
-    const int4 *q = reinterpret_cast<const int4 *>(e);
-    const int4 x = q[0], y = q[1], z = q[2];
-    SelEntry r;
-    r.it = (uint32_t)x.x;
-    r.q = (uint32_t)x.y;
-    r.ob = ((unsigned long long)(uint32_t)x.w << 32) | (uint32_t)x.z;
-    r.v = y.x;
-    r.s = y.y;
-    r.p = (uint32_t)y.z;
-    r.d = y.w;
-    r.beg = (long long)(((unsigned long long)(uint32_t)z.y << 32) | (uint32_t)z.x);
-    r.cls = z.z;
-    r.pad = z.w;
-    return r;
-}
-
-// Counted bytes of the prefix reads of one item (4 bytes per element staged
-// or probed): the staged entries, plus per draw the probes of the levels
-// searched in global memory (a 32-entry line: 5 probes each).
-__device__ __forceinline__ unsigned long long staged_bytes(const StagePlan &sp, int64_t d, int N) {
-    switch (sp.mode) {
-        case STAGE_ROW: return 4ull * d;
-        case STAGE_CDF1: return 4ull * sp.count + (unsigned long long)N * 4ull * 5;
-        case STAGE_CDF2: return 4ull * sp.count + (unsigned long long)N * 4ull * 10;
-        default: return (unsigned long long)N * 4ull * (64 - __clzll((unsigned long long)d));
-    }
-}
-
 // Level expansion, part 2 for items over a cached prefix with N <= 16 and
-// d >= 3N (a rebuild is rare): two items per warp, one per half-warp, lanes
-// N..15 of a half idle instead of N..31 of a warp.  For each item the bulk
-// copy engine stages, on one barrier: its work entry, the 16 bytes holding
-// its prefix total T, and what its draws search (stage_plan: the prefix row
-// up to WF edges, else the row's entries of the first or second prefix index
-// level).  The next item's copies are requested as soon as the current
-// item's draws are resolved, so they overlap the current item's edge
-// emission (dependent neighbor-record gathers and stores).  Every draw
-// searches the staged array in shared memory by fixed-step lifting; index
-// entries then lead to one 32-entry line per remaining level in global
-// memory, so rows and hubs share one resolver loop.  Items that need a
-// rebuild go on from their failed first phase (its state kept in the
-// consumed pair entry): rows up to WF edges by k_select_fast on the refill
-// list (written over the consumed warp list), larger ones by the CTA pass.
-constexpr int PAIR_ENT = 16;   // floats of a half's entry slot: the 48-byte entry and the 16-byte T window
-
+// d >= 3N (a rebuild is rare): 32 / N items per warp, slot s of the warp's
+// item i on lane i * N + s.  All items of a warp run the same instructions:
+// their entries, first draws and searches (cdf_find), then rounds as in
+// resolve_slots -- one match over the warp finds every repeated candidate,
+// each item's lanes look at their own, and the repeats of all items draw
+// again together -- until no item has one.  Items that need a rebuild go on
+// from their failed first phase (its state kept in the consumed entry): rows
+// up to WF edges by k_select_fast on the refill list (written over the
+// consumed warp list), larger ones by the CTA pass.
+//
+// What bounds it: dependent sector gathers (entry, total and tile line, edge
+// line, column) and the instructions of the rounds, about equally: 47% issue
+// active, 3.8 TB/s of DRAM, 19 cycles between a warp's instructions, 11 of
+// them waiting for loads (level 2 at R-MAT scale 22).  An item costs 270 warp
+// instructions; two items a warp in halves of their own, their rows staged
+// in shared memory by the bulk copy engine, cost 550, as the halves diverged
+// in draws and refinements and paid the staging per item.  The gathers need
+// no shared memory, so registers set the occupancy: 40 a thread, six CTAs
+// (48 and five: 4% slower), which is why a slot's later draw words and the
+// recording clock wait in shared memory and the entry is read again when its
+// edges are emitted.  Scale-25 step: 23.4 -> 18.4 ms; an 8192-seed [15,10,5]
+// request on R-MAT 22: 0.55 -> 0.43 ms.
 template <typename I, int BIAS>
-__device__ __forceinline__ void pair_body(const DevGraph &g, const LevelArgs &a, float *buf, float *ebuf,
-                                          uint64_t *bar, uint32_t &parity) {
+__device__ __forceinline__ void group_body(const DevGraph &g, const LevelArgs &a) {
+    static_assert(REJECT_ATTEMPTS == 4, "a first phase's draws are one Philox block");
+    __shared__ uint32_t s_word[3 * FAST_THREADS];        // per thread: its slot's draws 1..3 of the phase
+    __shared__ long long s_t0[FAST_THREADS / 32];        // recording: when the warp's items began
     const int lane = threadIdx.x & 31;
-    const Half h(lane);
-    const uint32_t gh = (blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-    const uint32_t nh = (gridDim.x * blockDim.x) >> 4;
+    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint32_t n = __ldcg(a.n_pair);
-    const uint32_t n_level = __ldcg(a.n_in);
     const int N = a.N;
     const int nout = 2 + (a.o_smp != nullptr) + (a.o_dep != nullptr);
-    unsigned long long my_bytes = 0;
-    uint32_t my_items = 0;   // at most n per lane
-    // requests the staged copies of item idx (row range rbeg, rd); returns the
-    // offset of its staged array in the buffer
-    auto request = [&](uint32_t idx, long long rbeg, int rd) -> int {
-        const StagePlan sp = stage_plan(g, rbeg, rd);
-        RowWindow w{nullptr, 0, 0u};
-        if (sp.mode != STAGE_NONE) w = row_window(sp.src, sp.count);
-        if (h.sl == 0) {
-            const int64_t e = rbeg + rd - 1;   // T's element; the cache is padded past its last row
-            fence_async_smem();                // this half's reads of buf precede the copies' writes
-            bulk_load3(ebuf, a.pair_list + idx, (uint32_t)sizeof(SelEntry), ebuf + 12, g.cdf + (e & ~(int64_t)3), 16u,
-                       buf, w.start, w.bytes, bar);
-        }
-        return w.off;
-    };
-    // The item loop is uniform across the warp (half h takes item base + h;
-    // on the warp's last item the second half may idle), so the two halves
-    // meet at a full-warp barrier after their draws and run the copy
-    // request, the emission and the bookkeeping as one instruction stream.
-    const uint32_t hw = lane >> 4;
-    const uint32_t wstep = nh;   // two halves per warp
-    uint32_t i = gh;
-    bool dead = false;           // a copy wait expired: this half stops
-    int off = 0;
-    if (i < n) off = request(i, __ldcg(&a.pair_list[i].beg), __ldcg(&a.pair_list[i].d));
-    for (uint32_t base = gh - hw; base < n; base += wstep, i += wstep) {
-        const bool act = i < n && !dead;
-        const uint32_t inext = i + wstep;
-        long long nbeg = 0;
-        int nd = 0;
-        if (act && inext < n) {   // the next item's range: its load overlaps this item
-            nbeg = __ldcg(&a.pair_list[inext].beg);
-            nd = __ldcg(&a.pair_list[inext].d);
-        }
-        int jfail = -1;   // -1: all slots accepted; else the slot whose first phase failed
-        SelEntry en{};
-        StagePlan sp{STAGE_NONE, nullptr, 0};
-        int sel = 0;
-        long long t0 = 0;
-        const bool rec = a.sched && a.sched->mode == SCHED_RECORD;
+    const uint32_t G = 32 / N;
+    const uint32_t gi = (uint32_t)lane / (uint32_t)N;
+    const int first = (int)gi * N, sl = lane - first;   // the item's first lane, the lane's slot
+    const unsigned gmask = gi < G ? (N == 32 ? FULL : ((1u << N) - 1u)) << first : 0u;
+    const unsigned below = gmask & ((1u << lane) - 1u);
+    const bool rec = a.sched && a.sched->mode == SCHED_RECORD;
+    uint32_t my_items = 0, my_probes = 0;
+#pragma unroll 1
+    for (uint32_t base = gw * G; base < n; base += nw * G) {
+        const uint32_t i = base + gi;
+        bool act = gi < G && i < n;
+        if (rec && lane == 0) s_t0[threadIdx.x >> 5] = clock64();
+        // what the draws need of the entry; the rest is read again when the
+        // edges are emitted, so it does not hold registers over the search
+        int64_t beg = 0;
+        int d = 0;
+        float T = 0.f;
+        uint32_t x = 0;
+        int cand = -2 - lane, used = 0;
         if (act) {
-            if (!mbar_wait(bar, parity)) {   // bounded: report instead of spinning on
-                if (h.sl == 0) atomicOr(a.err, ERR_COPY_WAIT);
-                mbar_wait(bar, parity);        // let the copies in flight land first
-                dead = true;
-            } else {
-                parity ^= 1u;
+            const int4 *q = reinterpret_cast<const int4 *>(a.pair_list + i);
+            const int4 y = __ldcg(q + 1);
+            beg = __ldcg(reinterpret_cast<const long long *>(q + 2));
+            d = y.w;
+            T = __ldg(g.cdf + beg + d - 1);
+            // the slot's draws of the first phase are one block's words
+            const uint4 blk = philox(make_uint4((uint32_t)y.z, (uint32_t)y.y, (TAG_SAMPLE << 24) | (uint32_t)a.depth,
+                                                (uint32_t)sl << 16), a.k0, a.k1);
+            x = blk.x;
+            s_word[threadIdx.x] = blk.y;
+            s_word[FAST_THREADS + threadIdx.x] = blk.z;
+            s_word[2 * FAST_THREADS + threadIdx.x] = blk.w;
+        }
+        bool draw = act;
+#pragma unroll 1
+        for (;;) {
+            if (draw) {
+                if (used) x = s_word[(used - 1) * FAST_THREADS + threadIdx.x];
+                cand = cdf_find(g, beg, d, x, T);
+                if (!(T > 0.f)) cand = sl;   // no mass: the slots take indices 0..N-1
+                ++used;
+            }
+            // lanes of the item holding the same candidate, before this one;
+            // an accepted slot never has any, so the first slot with one is
+            // the item's current slot and the slots before it are accepted
+            const unsigned lower = __match_any_sync(FULL, cand) & below;
+            const unsigned db = __ballot_sync(FULL, lower != 0u);
+            if (db == 0u) break;
+            const unsigned mine = db & gmask;
+            const int f = __ffs(mine) - 1;   // -1: the item is done
+            draw = (lower & ((1u << (f & 31)) - 1u)) != 0u && used < REJECT_ATTEMPTS;
+            const unsigned ab = __ballot_sync(FULL, draw);
+            if (mine && !((ab >> f) & 1u)) {
+                // slot f's draws of the first phase ran out: a whole warp
+                // (rows) or CTA (hubs) rebuilds the prefix and goes on.  The
+                // failing slot and the accepted indices (16-bit) go into the
+                // item's entry, which nothing reads any more.
+                const bool keep = d <= RESUME_MAX_DEG && i < 0x7FFFFFFFu;
+                if (sl == 0) {
+                    const int4 *q = reinterpret_cast<const int4 *>(a.pair_list + i);
+                    int4 *o = reinterpret_cast<int4 *>(
+                        d <= WF ? a.refill_list + atomicAdd(a.n_refill, 1u) : a.retry_list + atomicAdd(a.n_retry, 1u));
+                    o[0] = __ldcg(q);
+                    o[1] = __ldcg(q + 1);
+                    int4 z = __ldcg(q + 2);
+                    if (keep) z.w = (int)(i + 1);   // pad: where its first phase's state waits
+                    o[2] = z;
+                }
+                __syncwarp(gmask);   // the entry is read before its first bytes are overwritten
+                if (keep) {
+                    uint16_t *ps = reinterpret_cast<uint16_t *>(a.pair_list + i);
+                    if (lane < f) ps[1 + sl] = (uint16_t)cand;
+                    if (sl == 0) ps[0] = (uint16_t)(f - first);
+                }
+                act = draw = false;
+                cand = -2 - lane;
             }
         }
-        const bool run = act && !dead;
-        if (run) {
-            en = load_sel_smem(reinterpret_cast<const SelEntry *>(ebuf));
-            const int64_t beg = en.beg, d = en.d;
-            const float T = ebuf[12 + ((beg + d - 1) & 3)];
-            const DrawCtx dc{a.k0, a.k1, en.p, (uint32_t)en.s, (uint32_t)a.depth};
-            if (rec) t0 = clock64();
-            sp = stage_plan(g, beg, (int)d);
-            const float *S = buf + off;   // the staged row or index entries
-            jfail = half_select(h, N, dc, T, [&](uint32_t x) -> int {
-                const float t = its_target(x, T);
-                if (sp.mode == STAGE_NONE) return (int)cdf_search(g, beg, d, t);
-                const int r = search_upper_lift<9>(S, sp.count, t);
-                return sp.mode == STAGE_ROW ? r : (int)staged_refine(g, sp.mode, r, beg, d, t);
-            }, sel);
+        if (act) {
+            const SelEntry en = load_sel(a.pair_list + i);
+            emit_edge<I>(g, a, beg + cand, en.v, en.s, en.p * (uint32_t)N + (uint32_t)sl, (int64_t)en.ob + sl,
+                         en.q + (uint32_t)sl);
+            if (sl == 0) {
+                ++my_items;
+                my_probes += 32 - __clz(d);
+            }
         }
-        const bool ok = jfail < 0;
-        __syncwarp();   // both halves: every read of the buffers is done, they are free
-        if (run && inext < n) off = request(inext, nbeg, nd);
-        const bool keep = en.d <= RESUME_MAX_DEG && i < 0x7FFFFFFFu;
-        if (run && !ok && keep) {
-            // a whole warp (rows) or CTA (hubs) goes on from the failed first
-            // phase: the failing slot and the accepted indices (16-bit) go
-            // into this item's pair entry, which nothing reads after its copy
-            // has landed
-            uint16_t *ps = reinterpret_cast<uint16_t *>(a.pair_list + i);
-            if (h.sl < jfail) ps[1 + h.sl] = (uint16_t)sel;
-            if (h.sl == 0) ps[0] = (uint16_t)jfail;
-        }
-        if (run && !ok && h.sl == 0) {   // rebuild needed: a whole warp or CTA goes on with the item
-            if (keep) en.pad = (int32_t)(i + 1);   // where its first phase's state waits
-            if (en.d <= WF) a.refill_list[atomicAdd(a.n_refill, 1u)] = en;
-            else a.retry_list[atomicAdd(a.n_retry, 1u)] = en;
-        }
-        if (run && ok && h.sl < N)
-            emit_edge<I>(g, a, en.beg + sel, en.v, en.s, en.p * (uint32_t)N + (uint32_t)h.sl, (int64_t)en.ob + h.sl,
-                         en.q + (uint32_t)h.sl);
-        if (run && ok && rec) {
-            __syncwarp(h.mask);
-            if (h.sl == 0)
-                record_profile(a.sched, en.d, N, a.sched->vstats[en.v], n_level, a.depth, en.cls, clock64() - t0);
-        }
-        if (run && ok && h.sl == 0) {
-            my_items++;
-            const unsigned long long row = staged_bytes(sp, en.d, N);
-            my_bytes += 16 + row + (unsigned long long)N * (4ull + 4ull * nout +
-                                                            (a.push ? 12ull + 2 * (sizeof(I) + 4) : 0ull));
+        if (rec) {
+            __syncwarp();
+            if (act && sl == 0) {
+                const SelEntry en = load_sel(a.pair_list + i);
+                record_profile(a.sched, d, N, a.sched->vstats[en.v], __ldcg(a.n_in), a.depth, en.cls,
+                               clock64() - s_t0[threadIdx.x >> 5]);
+            }
+            __syncwarp();
         }
     }
+    // counted bytes: per item its entry's 16, per draw one 4-byte prefix probe
+    // per halving of the row and the edge's records
+    unsigned long long my_bytes = (unsigned long long)my_probes * N * 4ull +
+                                  (unsigned long long)my_items *
+                                      (16ull + (unsigned long long)N * (4ull + 4ull * nout +
+                                                                        (a.push ? 12ull + 2 * (sizeof(I) + 4) : 0ull)));
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
         my_bytes += __shfl_xor_sync(FULL, my_bytes, o);
@@ -1076,28 +937,15 @@ __device__ __forceinline__ void pair_body(const DevGraph &g, const LevelArgs &a,
     }
 }
 
-// Shared staging buffers of the pair pass: one row window and one entry slot
-// per half-warp, each half with its bulk-copy barrier.
-constexpr int PAIR_HALVES = FAST_THREADS / 16;
-constexpr int PAIR_ROW = WF + 4;   // floats: a row of up to WF plus its 16-byte alignment window
-
 template <typename I, int BIAS>
-__global__ void __launch_bounds__(FAST_THREADS, CSAW_PAIR_MIN_BLOCKS)
-k_select_pair(DevGraph g, LevelArgs a) {
-    __shared__ __align__(16) float s_P[PAIR_HALVES * PAIR_ROW];
-    __shared__ __align__(16) float s_E[PAIR_HALVES * PAIR_ENT];
-    __shared__ __align__(8) uint64_t s_bar[PAIR_HALVES];
-    const int hid = threadIdx.x >> 4;
-    if ((threadIdx.x & 15) == 0) mbar_init(s_bar + hid);
-    mbar_init_fence();
-    __syncthreads();
-    uint32_t parity = 0;
-    pair_body<I, BIAS>(g, a, s_P + hid * PAIR_ROW, s_E + hid * PAIR_ENT, s_bar + hid, parity);
+__global__ void __launch_bounds__(FAST_THREADS, CSAW_GROUP_MIN_BLOCKS)
+k_select_group(DevGraph g, LevelArgs a) {
+    group_body<I, BIAS>(g, a);
 }
 
 // Level expansion, part 2 for hub items (d > WF) over a cached prefix: one
 // warp per item, each draw a search of the prefix through its index
-// (cdf_search) taken one attempt at a time, since a search costs dependent
+// (cdf_find) taken one attempt at a time, since a search costs dependent
 // loads; no shared memory.  An item whose draws need a rebuild of its prefix
 // goes to the retry list (the CTA pass rebuilds it in global scratch).
 template <typename I, int BIAS>
@@ -1348,7 +1196,8 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
                     uint4 b = philox(make_uint4(0u, (uint32_t)(a.base + w), (TAG_SAMPLE << 24) | (uint32_t)t, 0u), a.k0, a.k1);
                     if constexpr (BIASED) {
                         const float T = __ldg(g.cdf + beg + d - 1);
-                        if (T > 0.f) idx = (uint32_t)cdf_search(g, beg, d, its_target(b.x, T));
+                        idx = (uint32_t)cdf_find(g, beg, d, b.x, T);
+                        if (!(T > 0.f)) idx = 0;
                         probes += 1 + (64 - __clzll((unsigned long long)d));
                     } else {
                         idx = mulhi(b.x, (uint32_t)d);

@@ -82,11 +82,6 @@ __device__ __forceinline__ void grid_barrier(unsigned *arrive, unsigned nblocks,
     __syncthreads();
 }
 
-// Bytes of dynamic shared memory of k_persist: the pair pass's row windows,
-// entry slots and barriers.
-constexpr size_t PERSIST_SMEM =
-    sizeof(float) * PAIR_HALVES * (PAIR_ROW + PAIR_ENT) + sizeof(uint64_t) * PAIR_HALVES;
-
 // The passes: the frequent ones inlined into the one kernel, the hub and
 // CTA-retry passes (rare, with large state of their own) as calls, so their
 // registers do not weigh on the inlined loops.
@@ -103,9 +98,8 @@ __device__ __noinline__ void call_hub(const DevGraph &g, const LevelArgs &a) {
     hub_body<I, BIAS>(g, a);
 }
 template <typename I, int BIAS>
-__device__ __forceinline__ void call_pair(const DevGraph &g, const LevelArgs &a, float *buf, float *ebuf,
-                                       uint64_t *bar, uint32_t &parity) {
-    pair_body<I, BIAS>(g, a, buf, ebuf, bar, parity);
+__device__ __forceinline__ void call_group(const DevGraph &g, const LevelArgs &a) {
+    group_body<I, BIAS>(g, a);
 }
 template <typename I, int BIAS>
 __device__ __noinline__ void call_heavy(const DevGraph &g, const LevelArgs &a) {
@@ -120,17 +114,6 @@ template <typename I, int BIAS>
 __global__ void __launch_bounds__(FAST_THREADS, CSAW_PERSIST_MIN_BLOCKS)
 k_persist(const __grid_constant__ DevGraph g, const __grid_constant__ PersistArgs pa) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
-    extern __shared__ float s_heavy[];   // the same dynamic region heavy_body names (unused by it here)
-    float *pairP = s_heavy;
-    float *pairE = s_heavy + PAIR_HALVES * PAIR_ROW;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(pairE + PAIR_HALVES * PAIR_ENT);
-    const int hid = threadIdx.x >> 4;
-    if (BIASED) {
-        if ((threadIdx.x & 15) == 0) mbar_init(bars + hid);
-        mbar_init_fence();
-    }
-    __syncthreads();
-    uint32_t parity = 0;
     const unsigned nblocks = gridDim.x;
     int k = 0;
     for (int l = 0; l < pa.D; ++l) {
@@ -139,8 +122,7 @@ k_persist(const __grid_constant__ DevGraph g, const __grid_constant__ PersistArg
         grid_barrier(pa.arrive + k++, nblocks, pa.err);
         call_select<I, BIAS, BIASED>(g, pa.lv[l]);
         if (fl & PF_HUB) call_hub<I, BIAS>(g, pa.lv[l]);
-        if (BIASED && (fl & PF_PAIR))
-            call_pair<I, BIAS>(g, pa.lv[l], pairP + hid * PAIR_ROW, pairE + hid * PAIR_ENT, bars + hid, parity);
+        if (BIASED && (fl & PF_PAIR)) call_group<I, BIAS>(g, pa.lv[l]);
         grid_barrier(pa.arrive + k++, nblocks, pa.err);
         if (BIASED && (fl & PF_PAIR)) call_select<I, BIAS, true>(g, pa.refill[l]);
         if (fl & PF_RETRY) {

@@ -100,8 +100,7 @@ __device__ __forceinline__ int select_warp(const DevGraph &g, int64_t beg, int64
     auto cand_of = [&](uint32_t x, bool act) -> int {
         if (!act) return -1;
         if constexpr (BIASED) {
-            const float t = its_target(x, T);
-            return indexed ? (int)cdf_search(g, beg, d, t) : (int)search_upper(P, d, t);
+            return indexed ? cdf_find(g, beg, (int)d, x, T) : (int)search_upper(P, d, its_target(x, T));
         } else {
             return kth_not_excluded(mulhi(x, (uint32_t)(d - nZ)), zs, nZ);
         }
@@ -475,17 +474,104 @@ __device__ __forceinline__ int incr_search(WFn wfn, int64_t d, const int32_t *zs
     return res;
 }
 
-// One CTA per deferred item: the canonical prefix is built by the whole CTA in
-// shared memory when the launch has room for the row (a.heavy_smem), else in
-// global scratch (same canonical order, so bit-identical to the warp path);
-// warp 0 runs the slot resolver; a rebuild is incremental over the tile
-// summaries for a cached hub (incr_rebuild), else a CTA-wide rescan.
+// Shared state of a CTA that runs one item (heavy_select).
+struct HeavyShared {
+    int flag, j, nz;
+    int32_t z[32];              // zeroed neighbors of an incremental rebuild
+    float gm[INCR_SGROUPS];     // its group maxima
+    float row[32 * 33];         // its draws' staged tiles
+};
+
+// Selection for one item by the whole CTA (all threads call it): a canonical
+// prefix that has to be computed is built by every warp in P (shared memory
+// or global scratch of heavy_need(d) floats; the same canonical order, so
+// bit-identical to the warp path); warp 0 runs the slot resolver; a rebuild
+// is incremental over the tile summaries for a cached hub (incr_rebuild),
+// else a CTA-wide rescan.  j0 > 0 resumes an item over a cached prefix whose
+// first phase failed at slot j0 (warp 0's lane m < j0 passes its accepted
+// index in sel0): a rebuild without the j0 selections, slot j0 from draw
+// REJECT_ATTEMPTS.  Returns the lane's selection (warp 0's lanes < N); adds
+// the counted prefix reads of the rebuilds to rebuild_bytes.
+template <typename I, int BIAS, bool STREAM>
+__device__ __forceinline__ int heavy_select(const DevGraph &g, int32_t v, int64_t beg, int64_t d, int N,
+                                            const DrawCtx &dc, float *P, HeavyShared &sh, int j0, int sel0,
+                                            unsigned long long &rebuild_bytes) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *tsum = P + d;
+    float *gcar = tsum + (d >> 5) + 1;
+    uint32_t *zb = (uint32_t *)(gcar + (d >> 10) + 1);
+    auto wfn = [&](int64_t i) { return edge_bias<I, BIAS>(g, beg + i); };
+    bool indexed = g.cdf && g.cdf_bias == BIAS;   // cached prefix, searched through its index
+    // cached hub with tile summaries: rebuilds are incremental
+    const bool incr = !STREAM && indexed && g.tsc && d > TSC_MIN_DEG;
+    bool rebuilt = false;
+    const IncrView iv = incr_view(P, d);
+    float T = indexed ? g.cdf[beg + d - 1] : cta_canon_prefix(wfn, d, P, tsum, gcar, nullptr);
+    SlotRng rng;
+    SelState st;
+    auto cand_of = [&](uint32_t x, bool act) -> int {
+        const float t = act ? its_target(x, T) : 0.f;
+        if (rebuilt) return incr_search(wfn, d, sh.z, sh.nz, iv, sh.gm, sh.row, t, act, lane);   // all lanes take part
+        if (!act) return -1;
+        return indexed ? cdf_find(g, beg, (int)d, x, T) : (int)search_upper(P, d, t);
+    };
+    bool zero = !(T > 0.f);
+    if (!indexed || zero || j0 >= N) j0 = 0;
+    if (warp == 0 && j0 > 0) {
+        st.j = j0;
+        if (lane < j0) st.sel = sel0;
+        if (lane == j0) st.A = REJECT_ATTEMPTS;
+    }
+    if (warp == 0 && !zero && j0 == 0) draw_pending(st, 0, N, lane, dc, rng, cand_of);
+    for (bool resumed = j0 > 0;; resumed = false) {
+        if (warp == 0) {
+            int r = 0;
+            if (resumed) r = 1;   // the rebuild after the failed first phase comes first
+            else if (zero) zero_fill(st, N, lane);
+            else r = resolve_slots(st, N, lane, dc, rng, cand_of);
+            if (lane == 0) {
+                sh.flag = r;
+                sh.j = st.j;
+            }
+        }
+        __syncthreads();
+        const int need = sh.flag, j = sh.j;
+        if (!need) break;
+        if (incr) {
+            if (warp == 0) {
+                if (lane < j) sh.z[lane] = st.sel;
+                if (lane == 0) sh.nz = j;
+            }
+            __syncthreads();
+            T = incr_rebuild(g, wfn, beg, v, d, sh.z, j, iv, sh.gm);
+            rebuilt = true;
+            // the row's tile summaries, the touched tiles' biases, and per
+            // later draw one line of running maxima and one tile of biases
+            rebuild_bytes += 8ull * (unsigned long long)iv.ntiles + 128ull * (unsigned long long)j +
+                             256ull * (unsigned long long)N;
+        } else {
+            const int64_t nwords = (d + 31) >> 5;
+            for (int64_t w = threadIdx.x; w < nwords; w += blockDim.x) zb[w] = 0u;
+            __syncthreads();
+            if (warp == 0 && lane < j) atomicOr(&zb[st.sel >> 5], 1u << (st.sel & 31));
+            __syncthreads();
+            T = cta_canon_prefix(wfn, d, P, tsum, gcar, zb);
+            rebuild_bytes += 4ull * (unsigned long long)d;   // every bias of the row again
+        }
+        indexed = false;
+        if (warp == 0) {
+            if (!(T > 0.f)) zero = true;
+            else draw_pending(st, j, N, lane, dc, rng, cand_of);
+        }
+    }
+    return st.sel;
+}
+
+// One CTA per deferred item (heavy_select), its prefix in shared memory when
+// the launch has room for the row (a.heavy_smem), else in global scratch.
 template <typename I, int BIAS, bool STREAM = false>
 __device__ __forceinline__ void heavy_body(const DevGraph &g0, const LevelArgs &a) {
-    __shared__ int s_flag, s_j, s_nz;
-    __shared__ int32_t s_z[32];                 // zeroed neighbors of an incremental rebuild
-    __shared__ float s_gm[INCR_SGROUPS];        // its group maxima
-    __shared__ float s_row[32 * 33];            // its draws' staged tiles
+    __shared__ HeavyShared sh;
     extern __shared__ float s_heavy[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float *const P_global = a.heavy_scratch + (int64_t)blockIdx.x * a.heavy_stride;
@@ -516,93 +602,28 @@ __device__ __forceinline__ void heavy_body(const DevGraph &g0, const LevelArgs &
             continue;
         }
         float *P = in_smem ? s_heavy : P_global;
-        float *tsum = P + d;
-        float *gcar = tsum + (d >> 5) + 1;
-        uint32_t *zb = (uint32_t *)(gcar + (d >> 10) + 1);
-        auto wfn = [&](int64_t i) { return edge_bias<I, BIAS>(g, beg + i); };
-        bool indexed = g.cdf && g.cdf_bias == BIAS;   // cached prefix, searched through its index
-        const bool indexed0 = indexed;
+        const bool indexed0 = g.cdf && g.cdf_bias == BIAS;
         unsigned long long rebuild_bytes = 0;         // counted prefix reads of the rebuilds
-        // cached hub with tile summaries: rebuilds are incremental
-        const bool incr = !STREAM && indexed && g.tsc && d > TSC_MIN_DEG;
-        bool rebuilt = false;
-        const IncrView iv = incr_view(P, d);
-        float T = indexed ? g.cdf[beg + d - 1] : cta_canon_prefix(wfn, d, P, tsum, gcar, nullptr);
         const DrawCtx dc{a.k0, a.k1, p, (uint32_t)s, (uint32_t)l};
-        SlotRng rng;
-        SelState st;
-        auto cand_of = [&](uint32_t x, bool act) -> int {
-            const float t = act ? its_target(x, T) : 0.f;
-            if (rebuilt) return incr_search(wfn, d, s_z, s_nz, iv, s_gm, s_row, t, act, lane);   // all lanes take part
-            if (!act) return -1;
-            return indexed ? (int)cdf_search(g, beg, d, t) : (int)search_upper(P, d, t);
-        };
-        bool zero = !(T > 0.f);
         // a pair item whose first phase failed at slot j0 (the entry's pad =
-        // its pair index + 1; the slot and the accepted indices wait in the
-        // consumed pair entry): the run goes on from there -- a rebuild
-        // without the j0 selections, slot j0 from draw REJECT_ATTEMPTS
-        int j0 = 0;
-        if (a.heavy_list && a.pair_list && indexed && !zero) {
+        // its pair index + 1): the slot and the accepted indices wait in the
+        // consumed pair entry
+        int j0 = 0, sel0 = -1;
+        if (a.heavy_list && a.pair_list) {
             const int pad = __ldcg(&a.heavy_list[h].pad);
             if (pad > 0 && d <= RESUME_MAX_DEG) {
                 const uint16_t *ps = reinterpret_cast<const uint16_t *>(a.pair_list + (pad - 1));
                 j0 = __ldcg(ps);
                 if (j0 >= N) j0 = 0;
-                if (warp == 0 && j0 > 0) {
-                    st.j = j0;
-                    if (lane < j0) st.sel = __ldcg(ps + 1 + lane);
-                    if (lane == j0) st.A = REJECT_ATTEMPTS;
-                }
+                if (warp == 0 && lane < j0) sel0 = __ldcg(ps + 1 + lane);
             }
         }
-        if (warp == 0 && !zero && j0 == 0) draw_pending(st, 0, N, lane, dc, rng, cand_of);
-        for (bool resumed = j0 > 0;; resumed = false) {
-            if (warp == 0) {
-                int r = 0;
-                if (resumed) r = 1;   // the rebuild after the failed first phase comes first
-                else if (zero) zero_fill(st, N, lane);
-                else r = resolve_slots(st, N, lane, dc, rng, cand_of);
-                if (lane == 0) {
-                    s_flag = r;
-                    s_j = st.j;
-                }
-            }
-            __syncthreads();
-            const int need = s_flag, j = s_j;
-            if (!need) break;
-            if (incr) {
-                if (warp == 0) {
-                    if (lane < j) s_z[lane] = st.sel;
-                    if (lane == 0) s_nz = j;
-                }
-                __syncthreads();
-                T = incr_rebuild(g, wfn, beg, v, d, s_z, j, iv, s_gm);
-                rebuilt = true;
-                // the row's tile summaries, the touched tiles' biases, and per
-                // later draw one line of running maxima and one tile of biases
-                rebuild_bytes += 8ull * (unsigned long long)iv.ntiles + 128ull * (unsigned long long)j +
-                                 256ull * (unsigned long long)N;
-            } else {
-                const int64_t nwords = (d + 31) >> 5;
-                for (int64_t w = threadIdx.x; w < nwords; w += blockDim.x) zb[w] = 0u;
-                __syncthreads();
-                if (warp == 0 && lane < j) atomicOr(&zb[st.sel >> 5], 1u << (st.sel & 31));
-                __syncthreads();
-                T = cta_canon_prefix(wfn, d, P, tsum, gcar, zb);
-                rebuild_bytes += 4ull * (unsigned long long)d;   // every bias of the row again
-            }
-            indexed = false;
-            if (warp == 0) {
-                if (!(T > 0.f)) zero = true;
-                else draw_pending(st, j, N, lane, dc, rng, cand_of);
-            }
-        }
+        const int sel = heavy_select<I, BIAS, STREAM>(g, v, beg, d, N, dc, P, sh, j0, sel0, rebuild_bytes);
         if (warp == 0) {
             bool act = lane < N;
             int32_t dst = 0;
             if (act) {
-                dst = Update(&g.v, __ldg(g.v.col + beg + st.sel), v);
+                dst = Update(&g.v, __ldg(g.v.col + beg + sel), v);
                 if (dst < 0 || dst >= g.v.n_vertices) {
                     atomicOr(a.err, ERR_UPDATE_RANGE);
                     dst = 0;

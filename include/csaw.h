@@ -141,7 +141,7 @@ int csaw_graph_stats(csaw_graph g, csaw_stats *out);
  * Kinds: 0 level expansion (batched: take-all pass), 1 high-degree (CTA)
  * expansion, 2 walk, 3 MDRW, 4 queue/seed/residency setup, 5 batched
  * warp-granularity selection pass, 6 batched hub selection (cached prefix),
- * 7 batched two-items-per-warp selection (cached prefix, N <= 16), 8 walk
+ * 7 batched selection of 32 / N items per warp (cached prefix, N <= 16), 8 walk
  * with one thread per walk (unbiased walks; many biased walks over a cached
  * prefix), 9 persistent job kernel (every level of a batched neighbor job in
  * one launch; its bytes and items are counted under the kinds of the passes
@@ -215,7 +215,7 @@ enum {
      * persistent grid size in percent of the occupancy-filled grid
      * (25..400, default 100) ... */
     CSAW_OPT_GRID_PCT = 3,
-    /* ... and whether cached items with N <= 16 run two per warp (1, the
+    /* ... and whether cached items with N <= 16 run 32 / N per warp (1, the
      * default) or one per warp (0). */
     CSAW_OPT_PAIR = 4,
     /* Host-buffer jobs (csaw_sample_host, host_buffers != 0) copy edges
