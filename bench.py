@@ -79,7 +79,7 @@ WORKLOADS = {
         text="(a) degree-biased neighbor sampling {na} samples F4 N20 D3 + (b) degree-biased random walks {nb} x 64"),
 }
 FLUSH_BYTES = 256 << 20
-KINDS = ("expand", "select", "select_thread", "hub", "pair", "heavy", "walk", "walk_thread", "setup")
+KINDS = ("expand", "select", "select_thread", "hub", "pair", "heavy", "walk", "walk_thread", "tree", "setup")
 TRAFFIC_TABLE = os.path.join(ROOT, "profiles", "dram_traffic_rmat22.md")
 
 
@@ -88,7 +88,7 @@ def kernel_name(kind, batched):
             "select_thread": "k_select_thread",
             "hub": "k_select_hub", "pair": "k_select_group", "heavy": "k_expand_heavy",
             "walk": "k_walk_fast" if batched else "k_walk_warp",
-            "walk_thread": "k_walk_thread_fast" if batched else "k_walk_thread", "setup": "setup"}[kind]
+            "walk_thread": "k_walk_thread_fast" if batched else "k_walk_thread", "tree": "k_tree", "setup": "setup"}[kind]
 
 
 def load_peaks():

@@ -24,6 +24,7 @@
 #include "csaw_internal.h"
 #include "kernels_fast.cuh"
 #include "kernels_persist.cuh"
+#include "kernels_tree.cuh"
 #include "sched_mlp.cuh"
 
 using namespace csaw;
@@ -54,7 +55,7 @@ int fail(int code, const std::string &msg) {
     } while (0)
 
 enum { KK_EXPAND = 0, KK_HEAVY = 1, KK_WALK = 2, KK_MDRW = 3, KK_INIT = 4, KK_SELECT = 5, KK_HUB = 6, KK_PAIR = 7,
-       KK_WALK_THREAD = 8, KK_PERSIST = 9, KK_SELECT_THREAD = 10, KK_COUNT = 11 };
+       KK_WALK_THREAD = 8, KK_PERSIST = 9, KK_SELECT_THREAD = 10, KK_TREE = 11, KK_COUNT = 12 };
 
 struct Counters {
     unsigned long long out_count;
@@ -470,6 +471,108 @@ void post_count(csaw_graph_s *g, JobCtx *c, cudaStream_t st) {
     k_post_count<<<1, 1, 0, st>>>(&c->ctr->out_count, &c->posts[c->n_posts++]);
 }
 
+// Neighbor jobs whose sample trees run whole in one launch (k_tree): those
+// whose frontier levels hold at most this many items, counted by their bound
+// (FrontierSize x the fan-outs).  Below it the per-level launches are most of
+// a job's time; above it a chunk's levels, one after another on one SM, cost
+// more than launches that spread every level over the GPU.  Per-level passes
+// and one launch, us a call on a B200: 64 seeds [25,10] 123 and 69, 1024 148
+// and 78, 8192 (213 K items by the bound) 215 and 176, 16384 (426 K) 243 and
+// 265; 1024 seeds [15,10,5] (170 K) 245 and 129, 4096 (680 K) 329 and 500
+// (R-MAT 22, edge weights); F4 [20,20,20] on the power-law graph, 64 samples
+// (108 K) 128 and 92, 1024 (1.7 M) 173 and 239; unbiased [15,10], 16384 seeds
+// (262 K) 181 and 164; plain unbiased F4 [10,10], 8000 (352 K) 198 and 201.
+constexpr int64_t TREE_JOB_ITEMS = 1 << 18;
+
+template <typename I, int BIAS>
+bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], TreeArgs *t, int *threads) {
+    constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
+    const int S = p->n_samples, F = p->frontier_size, D = p->depth;
+    const bool plain = p->schedule == CSAW_SCHED_PLAIN;
+    if (BIASED && (plain || g->cdf_off)) return false;
+    if ((p->flags & CSAW_PARAM_DEDUP) && D > 1) return false;
+    if (D > TREE_MAX_LEVELS || g->E == 0) return false;
+    // launch-shape options keep the launches they shape
+    if (!plain && (g->persistent || g->grid_pct != 100 || !g->pair || g->thread_sel == 2)) return false;
+    if (p->schedule == CSAW_SCHED_LEARNED && BIASED) {   // only where the degree rule routes
+        const bool model = g->trained && (g->class_mask & 0x7cu) && !g->mlp_lost && !(g->trial && g->trial_arm == 0);
+        if (g->recording || model) return false;
+    }
+    double w = F, tot = 0;
+    uint32_t off[TREE_MAX_LEVELS + 1], wmax = 0;
+    for (int l = 0; l < D; ++l) {
+        if (w > TREE_MAX_ITEMS) return false;
+        off[l] = (uint32_t)tot;
+        wmax = std::max(wmax, (uint32_t)w);
+        tot += w;
+        w *= fan[l];
+    }
+    off[D] = (uint32_t)tot;
+    if (tot > TREE_MAX_ITEMS) return false;
+    if (tot * S > (double)TREE_JOB_ITEMS) return false;
+    // the widest CTAs (512 threads down to 128) whose chunks of one sample
+    // are all resident at once, 1024 threads an SM; more samples than that
+    // share chunks.  Us a call: 64 seeds [25,10] 69 at 512 threads, 79 at
+    // 128; 1024 seeds 79 at 128, 95 at 256 (two waves); 3001 unbiased [15,10]
+    // seeds 71 in chunks of 2 or 3, 80 in chunks of one
+    const int64_t room = 1024ll * g->sm_count;
+    int T = 512;
+    while (T > 128 && (int64_t)S * T > room) T >>= 1;
+    int C = (int)std::min<int64_t>(((int64_t)S * T + room - 1) / room, TREE_MAX_ITEMS);
+    C = std::min(C, (int)(TREE_MAX_ITEMS / tot));
+    t->per_chunk = C;
+    t->n_chunks = (S + C - 1) / C;
+    for (int l = 0; l <= D; ++l) t->qoff[l] = off[l] * (uint32_t)C;
+    t->wmax = wmax * (uint32_t)C;
+    *threads = T;
+    return true;
+}
+
+template <typename I, int BIAS>
+int run_tree(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int fan[], const int32_t *seeds,
+             const OutArgs &o, TreeArgs &t, int threads, cudaStream_t st) {
+    constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
+    const bool plain = p->schedule == CSAW_SCHED_PLAIN;
+    if (!plain) TRY(ensure_nbr(g, st));
+    if (BIASED) TRY((ensure_cdf<I, BIAS>(g, st)));
+    const TreeSmem m = tree_smem(threads / 32, t.qoff[p->depth], t.wmax, sizeof(I), BIASED);
+    static uint64_t attr_set = 0;   // per instantiation: bit = device
+    if (g->device < 64 && !((attr_set >> g->device) & 1u)) {
+        CK(cudaFuncSetAttribute(k_tree<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 << 10));
+        attr_set |= 1ull << g->device;
+    }
+    int64_t grid = std::min<int64_t>(t.n_chunks, grid_for(k_tree<I, BIAS>, threads, m.bytes, g->sm_count));
+    LevelArgs &a = t.lv;
+    if (BIASED && g->maxdeg > WF) {
+        a.heavy_stride = (g->maxdeg + 2 * ((g->maxdeg >> 5) + 1) + (g->maxdeg >> 10) + 1 + 8 + 63) & ~63ll;
+        grid = std::min<int64_t>(grid, std::max<int64_t>(1, SCRATCH_BUDGET / (a.heavy_stride * 4)));
+        TRY(ensure(c->hscratch, sizeof(float) * a.heavy_stride * grid, st));
+        a.heavy_scratch = (float *)c->hscratch.p;
+    }
+    a.o_src = o.src;
+    a.o_dst = o.dst;
+    a.o_smp = o.smp;
+    a.o_dep = o.dep;
+    a.o_count = o.count;
+    a.cap = o.cap;
+    a.bytes = c->ctr->bytes;
+    a.items = c->ctr->items;
+    a.err = &c->ctr->err;
+    a.k0 = (uint32_t)p->seed;
+    a.k1 = (uint32_t)(p->seed >> 32);
+    a.D = p->depth;
+    for (int l = 0; l < p->depth; ++l) a.fan[l] = (uint8_t)fan[l];
+    t.seeds = seeds;
+    t.n_samples = p->n_samples;
+    t.F = p->frontier_size;
+    t.base = (int)p->sample_base;
+    const DevGraph dg = dev_view(g, p->schedule, BIAS);
+    LaunchScope ls(g, KK_TREE, st);
+    k_tree<I, BIAS><<<(unsigned)grid, threads, m.bytes, st>>>(dg, t);
+    CK(cudaGetLastError());
+    return 0;
+}
+
 template <typename I, int BIAS>
 int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int fan[], const int32_t *seeds,
                    const OutArgs &o, cudaStream_t st) {
@@ -485,6 +588,11 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
         return fail(CSAW_ERR_INVALID, "FrontierSize * prod(NeighborSize) exceeds 2^32 lineage items");
     if (per_sample > (double)QUEUE_ITEM_BUDGET)
         return fail(CSAW_ERR_INVALID, "one sample's frontier exceeds the queue budget");
+    {
+        TreeArgs t{};
+        int threads = 0;
+        if (tree_shape<I, BIAS>(g, p, fan, &t, &threads)) return run_tree<I, BIAS>(g, c, p, fan, seeds, o, t, threads, st);
+    }
     int64_t B = (int64_t)((double)QUEUE_ITEM_BUDGET / per_sample);
     if (B > S) B = S;
     if (B < 1) B = 1;

@@ -303,13 +303,13 @@ __device__ __forceinline__ float warp_max_scan(float v, int lane) {
 // Passes of warp_canon_prefix over B tiles at once, tiles [t0, t0 + B) of
 // which the first `have` exist: the B shuffle chains are independent, so
 // their latencies (and the B bias loads) overlap.
-template <int B, typename WFn>
-__device__ __forceinline__ void canon_tiles_scan(WFn wfn, int64_t d, float *P, const uint32_t *zmask, int64_t t0,
+template <int B, typename D, typename WFn>
+__device__ __forceinline__ void canon_tiles_scan(WFn wfn, D d, float *P, const uint32_t *zmask, D t0,
                                                  int have, int slot, float &my_tsum, int lane) {
     float v[B];
 #pragma unroll
     for (int u = 0; u < B; ++u) {
-        const int64_t i = ((t0 + u) << 5) + lane;
+        const D i = ((t0 + u) << 5) + lane;
         v[u] = u < have && i < d ? wfn(i) : 0.f;
     }
     if (zmask) {
@@ -327,20 +327,20 @@ __device__ __forceinline__ void canon_tiles_scan(WFn wfn, int64_t d, float *P, c
     }
 #pragma unroll
     for (int u = 0; u < B; ++u) {
-        const int64_t i = ((t0 + u) << 5) + lane;
+        const D i = ((t0 + u) << 5) + lane;
         if (u < have && i < d) P[i] = v[u];
         const float s = __shfl_sync(FULL, v[u], 31);
         if (lane == slot + u) my_tsum = s;
     }
 }
 
-template <int B>
-__device__ __forceinline__ void canon_tiles_finish(int64_t d, float *P, int64_t t0, int have, int slot, float C,
+template <int B, typename D>
+__device__ __forceinline__ void canon_tiles_finish(D d, float *P, D t0, int have, int slot, float C,
                                                    float qex, float &runmax, int lane) {
     float p[B];
 #pragma unroll
     for (int u = 0; u < B; ++u) {
-        const int64_t i = ((t0 + u) << 5) + lane;
+        const D i = ((t0 + u) << 5) + lane;
         const float qx = __shfl_sync(FULL, qex, (slot + u) & 31);
         p[u] = u < have && i < d ? __fadd_rn(C, __fadd_rn(qx, P[i])) : 0.f;
     }
@@ -354,7 +354,7 @@ __device__ __forceinline__ void canon_tiles_finish(int64_t d, float *P, int64_t 
     }
 #pragma unroll
     for (int u = 0; u < B; ++u) {
-        const int64_t i = ((t0 + u) << 5) + lane;
+        const D i = ((t0 + u) << 5) + lane;
         p[u] = fmaxf(p[u], runmax);
         if (u < have && i < d) P[i] = p[u];
         if (u < have) runmax = __shfl_sync(FULL, p[u], 31);
@@ -366,12 +366,12 @@ __device__ __forceinline__ void canon_tiles_finish(int64_t d, float *P, int64_t 
 // every lane.  P may live in shared or global memory.  Four tiles at a time
 // (two where at most two are left): one tile after the other is a chain of
 // ten dependent shuffles and a load per tile, which made a rebuild of a
-// 512-edge row the longest part of a warp's item.
-template <typename WFn>
-__device__ float warp_canon_prefix(WFn wfn, int64_t d, float *P, const uint32_t *zmask, int lane) {
-    const int64_t ntiles = (d + 31) >> 5;
+// 512-edge row the longest part of a warp's item.  D: the row's index type.
+template <typename D, typename WFn>
+__device__ float warp_canon_prefix(WFn wfn, D d, float *P, const uint32_t *zmask, int lane) {
+    const D ntiles = (d + 31) >> 5;
     float C = 0.f, runmax = 0.f;
-    for (int64_t g0 = 0; g0 < ntiles; g0 += 32) {
+    for (D g0 = 0; g0 < ntiles; g0 += 32) {
         const int gt = (ntiles - g0) < 32 ? (int)(ntiles - g0) : 32;
         float my_tsum = 0.f;
         for (int tt = 0; tt < gt; tt += 4) {

@@ -294,6 +294,17 @@ template <typename I, int BIAS>
 __device__ __forceinline__ int select_cached(const DevGraph &g, int64_t beg, int d, int N, const DrawCtx &dc,
                                              float *P, uint32_t *zb, int lane, int j0 = 0, int sel0 = -1) {
     const float *cp = g.cdf + beg;
+    const bool lazy = d >= 4 * N;
+    // a row of few edges per slot needs rebuilds: its raw biases come to L2
+    // while the first phase runs
+    if constexpr (BIAS == CSAW_BIAS_EDGE_WEIGHT || BIAS == CSAW_BIAS_DEGREE) {
+        constexpr int PER_LINE = BIAS == CSAW_BIAS_EDGE_WEIGHT ? 32 : 8;
+        if (!lazy && lane * PER_LINE < d) {
+            const void *at = BIAS == CSAW_BIAS_EDGE_WEIGHT ? (const void *)(g.v.weight + beg + lane * PER_LINE)
+                                                           : (const void *)(g.nrec + beg + lane * PER_LINE);
+            if (BIAS == CSAW_BIAS_EDGE_WEIGHT || g.nrec) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+        }
+    }
     // a resumed item (j0 > 0) starts with a rebuild, which writes all of P
     for (int i0 = 0; i0 < (j0 > 0 ? 0 : d); i0 += 256) {
         float r[8];
@@ -323,7 +334,7 @@ __device__ __forceinline__ int select_cached(const DevGraph &g, int64_t beg, int
         T = warp_canon_prefix(wfn, d, P, zb, lane);
         return T > 0.f;
     };
-    return select_spec(N, lane, dc, !(T > 0.f), cand_of, rebuild, d >= 4 * N, j0, sel0);
+    return select_spec(N, lane, dc, !(T > 0.f), cand_of, rebuild, lazy, j0, sel0);
 }
 
 // Unbiased selection (no prefix): index ranks over the non-excluded range.
@@ -1110,7 +1121,7 @@ k_walk_fast(DevGraph g, WalkArgs a) {
                 }
                 float *buf = a.scratch + (int64_t)gw * a.scratch_stride;
                 auto wfn = [&](int64_t i) { return edge_bias<I, BIAS>(g, beg + i); };
-                const float T = warp_canon_prefix(wfn, d, buf, nullptr, lane);
+                const float T = warp_canon_prefix(wfn, (int64_t)d, buf, nullptr, lane);
                 e = beg + (T > 0.f ? search_upper(buf, d, its_target(x, T)) : 0);
                 bytes += (mat ? 4ull : 4ull + 2ull * sizeof(I)) * d;
             }

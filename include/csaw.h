@@ -53,8 +53,10 @@ enum {
 enum {
     CSAW_SCHED_PLAIN = 0,    /* one launch per level, degree-threshold rule */
     CSAW_SCHED_BATCHED = 1,  /* per-level passes by item class, CUDA-graph
-                                replayed; the one-launch persistent job
-                                kernel is CSAW_OPT_PERSISTENT */
+                                replayed; small and middle neighbor jobs run
+                                their sample trees in one launch; the
+                                one-launch persistent job kernel is
+                                CSAW_OPT_PERSISTENT */
     CSAW_SCHED_LEARNED = 2   /* batched + learned granularity */
 };
 
@@ -145,7 +147,9 @@ int csaw_graph_stats(csaw_graph g, csaw_stats *out);
  * with one thread per walk (unbiased walks; many biased walks over a cached
  * prefix), 9 persistent job kernel (every level of a batched neighbor job in
  * one launch; its bytes and items are counted under the kinds of the passes
- * it runs), 10 batched thread-per-item selection (N < d <= 32).
+ * it runs), 10 batched thread-per-item selection (N < d <= 32), 11 whole
+ * sample trees in one launch (small and middle neighbor jobs; its bytes and
+ * items too are counted under the kinds of the passes it stands for).
  */
 int csaw_graph_profile(csaw_graph g, int enable);
 int csaw_graph_kernel_stats(csaw_graph g, int kind, double *ms, int64_t *launches,
