@@ -154,6 +154,7 @@ struct JobCtx {
 
 struct csaw_graph_s {
     int device = 0, sm_count = 148;
+    int64_t l2_bytes = 126ll << 20;
     int64_t V = 0, E = 0, maxdeg = 0, n_non = 0;
     int idx64 = 0;
     void *rowptr = nullptr;
@@ -943,6 +944,16 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
     return 0;
 }
 
+// CTAs of `threads` threads for n walks of one thread each, at most gmax of
+// them: as many rounds as the resident threads need, each of the same size.
+// (A last round of a few walks takes as long as a full one's latency: 262,144
+// biased walks at 227,328 resident threads, R-MAT 22, 1.08 ms in a full and a
+// nearly empty round.)
+int even_grid(int64_t n, int threads, int gmax) {
+    const int64_t ctas = (n + threads - 1) / threads, rounds = (ctas + gmax - 1) / gmax;
+    return (int)std::max<int64_t>(1, (ctas + std::max<int64_t>(rounds, 1) - 1) / std::max<int64_t>(rounds, 1));
+}
+
 template <typename I, int BIAS>
 int run_walk_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *seeds, const OutArgs &o,
                cudaStream_t st) {
@@ -968,19 +979,30 @@ int run_walk_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
     a.k0 = (uint32_t)p->seed;
     a.k1 = (uint32_t)(p->seed >> 32);
     if (BIAS == CSAW_BIAS_UNBIASED) {
-        int grid = (p->n_samples + WALK_THREADS - 1) / WALK_THREADS;
-        int gmax = plain ? grid_for(k_walk_thread<I>, WALK_THREADS, 0, g->sm_count)
-                         : grid_for(k_walk_thread_fast<I, CSAW_BIAS_UNBIASED>, WALK_THREADS, 0, g->sm_count);
-        if (grid > gmax) grid = gmax;
+        // many unbiased walks are bound by their scattered sectors: where the
+        // 16-byte records are larger than L2 and the row offsets are not, the
+        // next row is read as a column and two offsets (an L2 hit more in the
+        // chain, but far fewer misses).  Us a call, walks of 40, records and
+        // columns: R-MAT 22, 65,536 walks 121 and 144, 100,000 155 and 153,
+        // 262,144 318 and 263; R-MAT 24 with 64-bit offsets (134 MB) 265 and
+        // 280; R-MAT 16 (records fit L2) 142 and 153.
+        a.by_col = !plain && p->n_samples >= 768ll * g->sm_count && (int64_t)sizeof(NbrRec) * g->E > g->l2_bytes &&
+                   (g->V + 1) * (int64_t)sizeof(I) <= g->l2_bytes / 2;
+        const int gmax = plain ? grid_for(k_walk_thread<I>, WALK_THREADS, 0, g->sm_count)
+                               : grid_for(k_walk_thread_fast<I, CSAW_BIAS_UNBIASED>, WALK_THREADS, 0, g->sm_count);
+        const int grid = even_grid(p->n_samples, WALK_THREADS, gmax);
         LaunchScope ls(g, KK_WALK_THREAD, st);
         if (plain) k_walk_thread<I><<<grid, WALK_THREADS, 0, st>>>(dg, a);
         else k_walk_thread_fast<I, CSAW_BIAS_UNBIASED><<<grid, WALK_THREADS, 0, st>>>(dg, a);
-    } else if (!plain && dg.cdf && (int64_t)p->n_samples >= 16ll * grid_for(k_walk_fast<I, BIAS>, FAST_THREADS, 0,
-                                                                               g->sm_count) * (FAST_THREADS / 32)) {
-        // many biased walks over a cached prefix: one thread per walk
-        int grid = (p->n_samples + WALK_THREADS - 1) / WALK_THREADS;
+    } else if (!plain && dg.cdf && (int64_t)p->n_samples >= 3ll * grid_for(k_walk_fast<I, BIAS>, FAST_THREADS, 0,
+                                                                              g->sm_count) * (FAST_THREADS / 32)) {
+        // many biased walks over a cached prefix: one thread per walk, from
+        // three walks per resident warp.  Us a call, walks of 40, a warp and a
+        // thread each: R-MAT 22 edge weights, 8192 walks 168 and 255, 16,384
+        // 305 and 266, 65,536 940 and 279; power-law graph, degree bias 105
+        // and 142, 175 and 154, 575 and 179
         const int gmax = grid_for(k_walk_thread_fast<I, BIAS>, WALK_THREADS, 0, g->sm_count);
-        if (grid > gmax) grid = gmax;
+        const int grid = even_grid(p->n_samples, WALK_THREADS, gmax);
         LaunchScope ls(g, KK_WALK_THREAD, st);
         k_walk_thread_fast<I, BIAS><<<grid, WALK_THREADS, 0, st>>>(dg, a);
     } else {
@@ -1330,6 +1352,8 @@ extern "C" int csaw_graph_create(const void *rowptr, int rowptr_is_64, const int
     auto *g = new csaw_graph_s();
     cudaGetDevice(&g->device);
     cudaDeviceGetAttribute(&g->sm_count, cudaDevAttrMultiProcessorCount, g->device);
+    int l2 = 0;
+    if (cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, g->device) == cudaSuccess && l2 > 0) g->l2_bytes = l2;
     {   // keep up to 2 GiB of freed stream-ordered workspace cached in the
         // device's default pool (process-local), so regrowth maps no memory
         cudaMemPool_t pool;

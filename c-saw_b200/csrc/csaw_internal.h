@@ -157,6 +157,7 @@ struct WalkArgs {
     int32_t *o_src, *o_dst, *o_smp, *o_dep;
     unsigned long long *o_count;
     int64_t cap;
+    int by_col;               // many walks: the next row from col and rowptr, not from the 16-byte record
     float *scratch;           // per-warp prefix scratch for d > WBUF (walks)
     int64_t scratch_stride;
     unsigned long long *bytes;

@@ -1028,6 +1028,7 @@ k_walk_fast(DevGraph g, WalkArgs a) {
     const unsigned long long obytes = 4ull * (2 + (a.o_smp != nullptr) + (a.o_dep != nullptr));
     const unsigned long long rec = 4ull + sizeof(I) + 4ull;   // col + neighbor record
     unsigned long long steps = 0, bytes = 0;
+    uint32_t rounds = 0;   // 5 x the 32-way search rounds of this warp's cached steps
     for (int w = gw; w < a.n; w += nw) {
         int32_t v = a.seeds[w];
         if (v < 0 || v >= g.v.n_vertices) {
@@ -1067,10 +1068,70 @@ k_walk_fast(DevGraph g, WalkArgs a) {
             int32_t u = 0, nd = 0;
             int64_t nb = 0;
             bool have = false;
-            bytes += obytes + rec;
             if (d == 1) {
             } else if (BIAS == CSAW_BIAS_UNBIASED) {
                 e = beg + mulhi(x, (uint32_t)d);
+            } else if (cached) {
+                // every round's probes are loaded together, the first round's
+                // with the total, the last round's with the records of the
+                // edges it decides between: one round trip for a row of one
+                // tile, two up to 1024 edges, three or four beyond
+                const float *cp = g.cdf + beg;
+                int lo = 0, n = d;        // the answer lies in row positions [lo, lo + n), n <= 32 at the end
+                float T, tt;
+                NbrRec r{};
+                float pv;
+                if (d <= 1024) {
+                    const int step = (d + 31) >> 5;
+                    const int at = (lane + 1) * step - 1 < d - 1 ? (lane + 1) * step - 1 : d - 1;
+                    pv = __ldg(cp + at);
+                    if (step == 1 && lane < d && g.nrec) r = load_rec(g.nrec, beg + lane);
+                    T = __shfl_sync(FULL, pv, 31);   // the last probe is the row's last entry
+                    tt = its_target(x, T);
+                    if (step > 1) {
+                        const int k = __ffs(__ballot_sync(FULL, at == d - 1 || pv > tt)) - 1;
+                        lo = k * step;
+                        n = d - lo < step ? d - lo : step;
+                    }
+                } else {
+                    const int o2 = (int)(beg & 1023), last = o2 + d - 1;   // the row's ends, from its first group
+                    const int64_t b0 = beg - o2;
+                    const int ng = (last >> 10) + 1;
+                    const float *c2 = g.cdf2 + (b0 >> 10);
+                    int u = 0, m = ng;
+                    T = __ldg(cp + d - 1);
+                    do {   // the last group's entry is never read: it is known to exceed the target
+                        const int st = (m + 31) >> 5, q = u + (lane + 1) * st - 1;
+                        pv = q < u + m - 1 ? __ldg(c2 + q) : 0.f;
+                        tt = its_target(x, T);
+                        const int k = __ffs(__ballot_sync(FULL, q >= u + m - 1 || pv > tt)) - 1;
+                        m = m - k * st < st ? m - k * st : st;
+                        u += k * st;
+                    } while (m > 1);
+                    const int ka = max(u << 5, o2 >> 5), kb = min((u << 5) + 31, last >> 5);   // its tiles
+                    const int q = ka + lane;
+                    pv = q < kb ? __ldg(g.cdf1 + (b0 >> 5) + q) : 0.f;
+                    const int k = ka + __ffs(__ballot_sync(FULL, q >= kb || pv > tt)) - 1;
+                    lo = max((k << 5) - o2, 0);
+                    n = min((k << 5) + 31, last) - o2 - lo + 1;
+                }
+                const bool mine = lane < n;
+                if (d > 32) {
+                    pv = mine ? __ldg(cp + lo + lane) : 0.f;
+                    if (mine && g.nrec) r = load_rec(g.nrec, beg + lo + lane);
+                }
+                int idx = __ffs(__ballot_sync(FULL, lane >= n - 1 || pv > tt)) - 1;
+                if (!(T > 0.f)) {   // no mass: the row's first edge
+                    idx = 0;
+                    lo = 0;
+                    if (g.nrec) r = load_rec(g.nrec, beg);
+                }
+                e = beg + lo + idx;
+                u = __shfl_sync(FULL, r.col, idx);
+                nb = __shfl_sync(FULL, r.beg, idx);
+                nd = __shfl_sync(FULL, r.deg, idx);
+                have = g.nrec != nullptr;
+                rounds += 36 - __clz(d);
             } else if (d <= 32) {
                 float wl = 0.f;
                 int32_t ul = 0, dl = 0;
@@ -1100,13 +1161,6 @@ k_walk_fast(DevGraph g, WalkArgs a) {
                 nd = __shfl_sync(FULL, dl, idx);
                 have = g.nrec != nullptr;
                 bytes += (mat ? 4ull : 4ull + 2ull * sizeof(I)) * d + rec * (d - 1);
-            } else if (cached) {
-                const float *cp = g.cdf + beg;
-                const float T = __ldg(cp + d - 1);
-                const float tt = its_target(x, T);
-                e = beg + (!(T > 0.f) ? 0 : (d > 1024 ? warp_cdf_search(g, beg, d, tt, lane)
-                                                       : warp_search_upper(cp, d, tt, lane)));
-                bytes += 4ull * 32 * ((68 - __clzll((unsigned long long)d)) / 5);   // 32 probes per round
             } else if (d <= WF) {
                 preload_bias<I, BIAS>(g, beg, d, W, lane);
                 auto wfn = [&](int64_t i) { return W[i]; };
@@ -1157,30 +1211,37 @@ k_walk_fast(DevGraph g, WalkArgs a) {
         flush();
     }
     if (lane == 0 && steps) {
-        atomicAdd(&a.bytes[2], bytes);
+        atomicAdd(&a.bytes[2], bytes + steps * (obytes + rec) + 128ull * (rounds / 5));   // 32 probes a round
         atomicAdd(&a.items[2], steps);
     }
 }
 
 // Walks with one thread per walk, for many walks: unbiased steps take one
 // round trip via the neighbor records; biased steps search the cached prefix
-// (the graph must hold it for BIAS) by binary search through its index, so a
-// warp keeps 32 walks in flight instead of one.  Same draws as the warp
-// kernels: step t of walk w uses word x of Philox(0, w, t).
+// (the graph must hold it for BIAS) through its index, so a warp keeps 32
+// walks in flight instead of one.  Same draws as the warp kernels: step t of
+// walk w uses word x of Philox(0, w, t).
+//
+// A step is a dependent gather or three, so nothing else may stand in a
+// walk's chain.  A thread keeps the vertices of WALK_KEEP steps in shared
+// memory; the warp then reserves their output range with one atomic and
+// writes them a step later, when the reservation has come back beside the
+// step's own loads.  (Staging 64 edges a warp and waiting for the atomic of
+// each flush took 531 us for 262,144 unbiased walks of 40 on R-MAT 22; this
+// takes 318, and 247 by columns: scattered 32-byte sectors, 40 G a second.)
+constexpr int WALK_KEEP = 8;
+
 template <typename I, int BIAS>
-__global__ void __launch_bounds__(WALK_THREADS)
+__global__ void __launch_bounds__(WALK_THREADS, BIAS == CSAW_BIAS_UNBIASED ? 8 : 6)
 k_walk_thread_fast(DevGraph g, WalkArgs a) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
-    __shared__ int32_t s_out[(WALK_THREADS / 32) * 4 * STAGE];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    WarpStage stg;
-    stg.s_src = s_out + wib * 4 * STAGE;
-    stg.s_dst = stg.s_src + STAGE;
-    stg.s_smp = stg.s_dst + STAGE;
-    stg.s_dep = stg.s_smp + STAGE;
-    const OutArgs oa{a.o_src, a.o_dst, a.o_smp, a.o_dep, a.o_count, a.cap};
+    __shared__ int32_t s_dst[WALK_KEEP * WALK_THREADS];   // [step][thread]
+    const int lane = threadIdx.x & 31;
+    int32_t *mine = s_dst + threadIdx.x;
     const int stride = gridDim.x * blockDim.x;
-    unsigned long long steps = 0, probes = 0;
+    unsigned long long steps = 0;
+    uint32_t probes = 0;   // of one walk at most a.len x 33
+    unsigned long long tot_probes = 0;
     for (int base = blockIdx.x * blockDim.x; base < a.n; base += stride) {
         const int w = base + threadIdx.x;
         bool alive = w < a.n;
@@ -1197,6 +1258,41 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
                 d = (int32_t)(row_begin<I>(g, v + 1) - beg);
             }
         }
+        int32_t first = v;                  // source of the kept steps' first edge
+        int kept = 0, t0 = 0;               // steps kept by this thread, the first one's number
+        unsigned long long out = 0;         // lane 0: the range reserved for them
+        // writes the kept steps of every lane, step by step
+        auto flush = [&]() {
+            unsigned long long pos0 = __shfl_sync(FULL, out, 0);
+            int32_t src = first;
+            for (int k = 0; k < WALK_KEEP; ++k) {
+                const unsigned m = __ballot_sync(FULL, k < kept);
+                if (m == 0u) break;
+                if (k < kept) {
+                    const int32_t dst = mine[k * WALK_THREADS];
+                    const int64_t pos = (int64_t)pos0 + __popc(m & ((1u << lane) - 1u));
+                    if (pos < a.cap) {
+                        a.o_src[pos] = src;
+                        a.o_dst[pos] = dst;
+                        if (a.o_smp) a.o_smp[pos] = a.base + w;
+                        if (a.o_dep) a.o_dep[pos] = t0 + k;
+                    }
+                    src = dst;
+                }
+                pos0 += __popc(m);
+            }
+        };
+        auto reserve = [&]() {
+            const unsigned n = __reduce_add_sync(FULL, (unsigned)kept);
+            if (lane == 0 && n) out = atomicAdd(a.o_count, (unsigned long long)n);
+        };
+        // the step's draw; unbiased, computed beside the load of the step before
+        // (biased walks have no register to hold it)
+        auto draw = [&](int t) -> uint32_t {
+            return philox(make_uint4(0u, (uint32_t)(a.base + w), (TAG_SAMPLE << 24) | (uint32_t)t, 0u), a.k0, a.k1).x;
+        };
+        uint32_t x = BIASED ? 0u : draw(0);
+        bool full = false;   // WALK_KEEP steps kept, their range reserved
         for (int t = 0; t < a.len; ++t) {
             if (alive && d <= 0) alive = false;
             if (!__any_sync(FULL, alive)) break;
@@ -1204,17 +1300,24 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
             if (alive) {
                 uint32_t idx = 0;
                 if (d > 1) {
-                    uint4 b = philox(make_uint4(0u, (uint32_t)(a.base + w), (TAG_SAMPLE << 24) | (uint32_t)t, 0u), a.k0, a.k1);
                     if constexpr (BIASED) {
                         const float T = __ldg(g.cdf + beg + d - 1);
-                        idx = (uint32_t)cdf_find(g, beg, d, b.x, T);
+                        idx = (uint32_t)cdf_find(g, beg, d, draw(t), T);
                         if (!(T > 0.f)) idx = 0;
-                        probes += 1 + (64 - __clzll((unsigned long long)d));
+                        probes += 33 - __clz(d);
                     } else {
-                        idx = mulhi(b.x, (uint32_t)d);
+                        idx = mulhi(x, (uint32_t)d);
                     }
                 }
-                const NbrRec r = edge_rec<I>(g, beg + idx);
+                NbrRec r;
+                if (a.by_col) {
+                    r.col = __ldg(g.v.col + beg + idx);
+                    r.beg = row_begin<I>(g, r.col);
+                    r.deg = (int32_t)(row_begin<I>(g, r.col + 1) - r.beg);
+                } else {
+                    r = edge_rec<I>(g, beg + idx);
+                }
+                if (!BIASED) x = draw(t + 1);
                 dst = Update(&g.v, r.col, v);
                 if (dst < 0 || dst >= g.v.n_vertices) {
                     atomicOr(a.err, ERR_UPDATE_RANGE);
@@ -1227,12 +1330,31 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
                 d = nd;
                 ++steps;
             }
-            stg.push(oa, alive, v, dst, a.base + w, t, lane);
-            if (alive) v = dst;
+            if (full) {
+                flush();
+                full = false;
+                kept = 0;
+                first = v;
+                t0 = t;
+            }
+            if (alive) {
+                mine[(t - t0) * WALK_THREADS] = dst;
+                ++kept;
+                v = dst;
+            }
+            if (t - t0 == WALK_KEEP - 1) {
+                reserve();
+                full = true;
+            }
+        }
+        if (!full) reserve();
+        flush();
+        if (BIASED) {
+            tot_probes += probes;
+            probes = 0;
         }
     }
-    stg.flush(oa, lane);
-    unsigned long long tot = steps, pr = probes;
+    unsigned long long tot = steps, pr = tot_probes;
     for (int off = 16; off; off >>= 1) {
         tot += __shfl_xor_sync(FULL, tot, off);
         pr += __shfl_xor_sync(FULL, pr, off);
