@@ -1046,7 +1046,15 @@ int run_mdrw_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
     a.err = &c->ctr->err;
     a.k0 = (uint32_t)p->seed;
     a.k1 = (uint32_t)(p->seed >> 32);
-    const size_t per_warp = (size_t)8 * a.F;
+    if (a.F <= 32) {
+        const int gmax = grid_for(k_mdrw_warp<I, BIAS>, WALK_THREADS, 0, g->sm_count);
+        const int grid = std::max(1, std::min((p->n_samples + WALK_THREADS / 32 - 1) / (WALK_THREADS / 32), gmax));
+        LaunchScope ls(g, KK_MDRW, st);
+        k_mdrw_warp<I, BIAS><<<grid, WALK_THREADS, 0, st>>>(dg, a);
+        CK(cudaGetLastError());
+        return 0;
+    }
+    const size_t per_warp = (size_t)12 * a.F;
     int wpb = (int)(96 * 1024 / per_warp);
     if (wpb > WALK_THREADS / 32) wpb = WALK_THREADS / 32;
     if (wpb < 1) wpb = 1;

@@ -1366,6 +1366,102 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
     }
 }
 
+// MDRW with a frontier of at most 32 vertices: one warp per sample, slot i on
+// lane i with its vertex, row and bias in registers.  A step's chain is the
+// neighbor's load alone where the graph has neighbor records (a column and
+// two row offsets otherwise): the biases of the unchanged slots, which a
+// frontier in shared memory gathered again every step, stay where they are,
+// lane l computes the draws of step t0 + l, and 32 steps' edges are written
+// together.  4000 samples F4 x 3: 18.6 -> 14.7 us on the device, 51 -> 48 a
+// call.
+template <typename I, int BIAS>
+__global__ void __launch_bounds__(WALK_THREADS)
+k_mdrw_warp(DevGraph g, WalkArgs a) {
+    const int lane = threadIdx.x & 31;
+    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int F = a.F;
+    unsigned long long steps = 0, visits = 0;
+    auto bias_of = [&](int32_t v, int32_t deg) -> float {
+        if constexpr (BIAS == CSAW_BIAS_UNBIASED) return 1.f;
+        else if constexpr (BIAS == CSAW_BIAS_DEGREE) return __int2float_rn(deg);
+        else return VertexBias(v, &g.v);
+    };
+    for (int s = gw; s < a.n; s += nw) {
+        int32_t v = 0, d = 0;
+        int64_t beg = 0;
+        float w = 0.f;
+        if (lane < F) {
+            v = a.seeds[(int64_t)s * F + lane];
+            if (v < 0 || v >= g.v.n_vertices) {
+                atomicOr(a.err, ERR_SEED_RANGE);
+                v = 0;
+            }
+            beg = row_begin<I>(g, v);
+            d = (int32_t)(row_begin<I>(g, v + 1) - beg);
+            w = bias_of(v, d);
+        }
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        int32_t rs = 0, rd = 0;   // lane l: the edge of step t0 + l, if it has one
+        bool have = false;
+        for (int t0 = 0; t0 < a.len; t0 += 32) {
+            x = philox(make_uint4(0u, (uint32_t)(a.base + s), (TAG_MDRW << 24) | (uint32_t)(t0 + lane), 0u), a.k0, a.k1);
+            have = false;
+            const int m = a.len - t0 < 32 ? a.len - t0 : 32;
+            for (int k = 0; k < m; ++k) {
+                int slot = 0;
+                if (F > 1) {
+                    const float P = tile_prefix(w, F, lane);
+                    const float T = __shfl_sync(FULL, P, 31);
+                    const float t = its_target(__shfl_sync(FULL, x.x, k), T);
+                    if (T > 0.f) slot = __ffs(__ballot_sync(FULL, lane >= F - 1 || P > t)) - 1;
+                }
+                const uint32_t y = __shfl_sync(FULL, x.y, k);
+                int32_t dst = 0;
+                const int32_t src = v;
+                if (lane == slot && d > 0) {
+                    const NbrRec r = edge_rec<I>(g, beg + mulhi(y, (uint32_t)d));
+                    dst = Update(&g.v, r.col, v);
+                    if (dst < 0 || dst >= g.v.n_vertices) {
+                        atomicOr(a.err, ERR_UPDATE_RANGE);
+                        dst = 0;
+                    }
+                    row_of<I>(g, r, dst, beg, d);
+                    v = dst;
+                    w = bias_of(v, d);
+                    ++steps;
+                    dst = ~dst;   // an edge (negative) or none (0)
+                }
+                const int32_t es = __shfl_sync(FULL, src, slot), ed = __shfl_sync(FULL, dst, slot);
+                if (lane == k) {
+                    rs = es;
+                    rd = ~ed;
+                    have = ed < 0;
+                }
+            }
+            visits += m;
+            const unsigned hm = __ballot_sync(FULL, have);
+            unsigned long long base = 0;
+            if (lane == 0 && hm) base = atomicAdd(a.o_count, (unsigned long long)__popc(hm));
+            base = __shfl_sync(FULL, base, 0);
+            const int64_t pos = (int64_t)base + __popc(hm & ((1u << lane) - 1u));
+            if (have && pos < a.cap) {
+                a.o_src[pos] = rs;
+                a.o_dst[pos] = rd;
+                if (a.o_smp) a.o_smp[pos] = a.base + s;
+                if (a.o_dep) a.o_dep[pos] = t0 + lane;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = 16; off; off >>= 1) steps += __shfl_xor_sync(FULL, steps, off);
+    if (lane == 0 && visits) {
+        // per step its slot's row range; per edge the neighbor and the edge written
+        atomicAdd(&a.bytes[3], visits * 2ull * sizeof(I) + steps * (4ull + 4ull * (2 + (a.o_smp != nullptr) + (a.o_dep != nullptr))));
+        atomicAdd(&a.items[3], steps);
+    }
+}
+
 template <typename I>
 __global__ void k_nbr_records(DevGraph g, NbrRec *rec) {
     const I *r = (const I *)g.v.rowptr;

@@ -831,8 +831,10 @@ k_walk_warp(DevGraph g, WalkArgs a) {
 }
 
 // ------------------------------------------------------------- MDRW
-// One warp per sample; frontier and its bias prefix in dynamic shared memory
-// (F ints + F floats per warp).
+// Frontiers above 32 vertices (smaller ones: k_mdrw_warp): one warp per sample;
+// frontier, its biases and their prefix in dynamic shared memory (F ints + 2 F
+// floats per warp).  A step changes one vertex, so the other biases are not
+// gathered again.
 template <typename I, int BIAS>
 __global__ void k_mdrw(DevGraph g, WalkArgs a) {
     extern __shared__ int32_t s_dyn[];
@@ -841,8 +843,13 @@ __global__ void k_mdrw(DevGraph g, WalkArgs a) {
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
     const int F = a.F;
-    int32_t *f = s_dyn + (int64_t)wib * 2 * F;
-    float *P = (float *)(f + F);
+    int32_t *f = s_dyn + (int64_t)wib * 3 * F;
+    float *P = (float *)(f + F), *W = P + F;
+    auto bias_of = [&](int32_t v) -> float {
+        if constexpr (BIAS == CSAW_BIAS_UNBIASED) return 1.f;
+        else if constexpr (BIAS == CSAW_BIAS_DEGREE) return degree_f<I>(g, v);
+        else return VertexBias(v, &g.v);
+    };
     WarpStage stg;
     stg.s_src = s_out + wib * 4 * STAGE;
     stg.s_dst = stg.s_src + STAGE;
@@ -859,20 +866,16 @@ __global__ void k_mdrw(DevGraph g, WalkArgs a) {
                 v = 0;
             }
             f[i] = v;
+            W[i] = bias_of(v);
         }
         __syncwarp();
         for (int t = 0; t < a.len; ++t) {
             uint4 b = philox(make_uint4(0u, (uint32_t)(a.base + s), (TAG_MDRW << 24) | (uint32_t)t, 0u), a.k0, a.k1);
             int slot = 0;
             if (F > 1) {
-                auto wfn = [&](int64_t i) -> float {
-                    if constexpr (BIAS == CSAW_BIAS_UNBIASED) return 1.f;
-                    else if constexpr (BIAS == CSAW_BIAS_DEGREE) return degree_f<I>(g, f[i]);
-                    else return VertexBias(f[i], &g.v);
-                };
+                auto wfn = [&](int i) -> float { return W[i]; };
                 float T = warp_canon_prefix(wfn, F, P, nullptr, lane);
                 if (T > 0.f) slot = (int)search_upper(P, F, its_target(b.x, T));
-                bytes += BIAS == CSAW_BIAS_UNBIASED ? 0 : 2ull * sizeof(I) * F;
             }
             const int32_t v = f[slot];
             const int64_t beg = row_begin<I>(g, v), d = row_begin<I>(g, v + 1) - beg;
@@ -887,7 +890,10 @@ __global__ void k_mdrw(DevGraph g, WalkArgs a) {
                 bytes += 4 + obytes;
                 ++steps;
                 __syncwarp();
-                if (lane == 0) f[slot] = dst;
+                if (lane == 0) {
+                    f[slot] = dst;
+                    W[slot] = bias_of(dst);
+                }
             }
             __syncwarp();
         }
