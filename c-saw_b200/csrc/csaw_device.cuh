@@ -268,6 +268,65 @@ __device__ __forceinline__ int cdf_find(const DevGraph &g, int64_t beg, int d, u
     return e0 + line_find(line, line_probes(line, a, b), a, b, t);
 }
 
+// cdf_find for a row whose prefix may lie in host memory (its index levels
+// and its total T are on the device): what counts there is the number of
+// 32-byte sectors asked for over the link.  The tile's end values are index
+// entries, so the target's place between them says which sector of the tile
+// line to ask for first; it decides, or its neighbor does.  One sector and a
+// half for uniform weights, where cdf_find asks for three or four and the
+// total is one more: R-MAT 24 through a 1 GiB budget, 18.4 -> 14.0 ms.  The
+// prefix has to be 32-byte aligned as its edges are numbered (host arrays
+// are; a partition's device copy need not be and is searched by cdf_find).
+__device__ __forceinline__ int cdf_find_far(const DevGraph &g, int64_t beg, int d, uint32_t x, float T) {
+    if ((reinterpret_cast<uintptr_t>(g.cdf) & 31) != 0) return cdf_find(g, beg, d, x, T);
+    const float t = its_target(x, T);
+    const int o2 = (int)(beg & 1023), last = o2 + d - 1;   // the row's ends, from its first group's start
+    const int64_t b0 = beg - o2;
+    int u = 0;
+    {
+        const float *c2 = g.cdf2 + (b0 >> 10);
+        int top = last >> 10;
+#pragma unroll 1
+        while (u < top) {
+            const int mid = (u + top) >> 1;
+            if (__ldg(c2 + mid) > t) top = mid; else u = mid + 1;
+        }
+    }
+    u <<= 5;
+    const float *c1 = g.cdf1 + (b0 >> 5);
+    const int kfirst = o2 >> 5, klast = last >> 5;
+    int lo = max(kfirst - u, 0), hi = min(klast - u, 31) + 1;
+    const int k = u + line_find(c1 + u, line_probes(c1 + u, lo, hi), lo, hi, t);
+    const float vlo = k > kfirst ? __ldg(c1 + k - 1) : 0.f, vhi = k < klast ? __ldg(c1 + k) : T;
+    const int e0 = k << 5;                                   // the tile, from b0
+    lo = max(o2 - e0, 0);
+    hi = min(last - e0, 31) + 1;                             // the answer lies in [lo, hi)
+    const float *line = g.cdf + b0 + e0;
+    int at = lo;
+    if (vhi > vlo) at += (int)(fminf(fmaxf((t - vlo) / (vhi - vlo), 0.f), 1.f) * (float)(hi - lo));
+    at = min(at, hi - 2);
+    while (lo < hi - 1) {   // entry hi - 1 is known to exceed t, those before lo not to
+        const int s = max(at, lo) & ~7, from = max(lo, s), to = min(hi - 1, s + 8);
+        float v[8];
+        asm("ld.global.nc.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+            : "l"(line + s));
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) c += s + i >= from && s + i < to && v[i] <= t ? 1 : 0;
+        if (from + c == to) {            // all at or below t
+            lo = at = to;
+        } else if (c > 0 || from == lo) {
+            lo = from + c;
+            break;
+        } else {                         // the first one read exceeds t: the sector before decides
+            hi = from + 1;
+            at = from - 1;
+        }
+    }
+    return e0 - o2 + lo;
+}
+
 // The same with one warp-uniform target, each level by warp_search_upper.
 __device__ __forceinline__ int64_t warp_cdf_search(const DevGraph &g, int64_t beg, int64_t d, float t, int lane) {
     const int64_t end = beg + d;

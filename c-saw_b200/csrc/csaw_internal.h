@@ -132,6 +132,7 @@ struct LevelArgs {
     // page-locked host weights.
     int part_cdf;
     const float *cdf1_all, *cdf2_all;
+    const float *row_total;   // per vertex, or null
     const float *host_w;
 };
 

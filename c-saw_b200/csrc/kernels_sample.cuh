@@ -77,11 +77,12 @@ static __global__ void k_init_queue(const int32_t *seeds, uint32_t n, int F, int
 // floats.  With a CDF cache the first phase searches the cached prefix, so d
 // may exceed cap; if such an item needs a phase rebuild (which must write a
 // prefix of d floats) every lane returns -2 and the caller hands the whole
-// item to the CTA path, which recomputes it with the same keys.
-template <typename I, int BIAS>
+// item to the CTA path, which recomputes it with the same keys.  FAR: the
+// prefix may lie in host memory; total: the row's, if known (else negative).
+template <typename I, int BIAS, bool FAR = false>
 __device__ __forceinline__ int select_warp(const DevGraph &g, int64_t beg, int64_t d, int N,
                                            const DrawCtx &dc, float *P, uint32_t *zb, int *zs,
-                                           int lane, int64_t cap) {
+                                           int lane, int64_t cap, float total = -1.f) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
     auto wfn = [&](int64_t i) { return edge_bias<I, BIAS>(g, beg + i); };
     float T = 0.f;
@@ -90,7 +91,7 @@ __device__ __forceinline__ int select_warp(const DevGraph &g, int64_t beg, int64
     if constexpr (BIASED) {
         if (g.cdf && g.cdf_bias == BIAS) {
             indexed = true;
-            T = g.cdf[beg + d - 1];
+            T = FAR && total >= 0.f ? total : g.cdf[beg + d - 1];
         } else {
             T = warp_canon_prefix(wfn, d, P, nullptr, lane);
         }
@@ -100,7 +101,8 @@ __device__ __forceinline__ int select_warp(const DevGraph &g, int64_t beg, int64
     auto cand_of = [&](uint32_t x, bool act) -> int {
         if (!act) return -1;
         if constexpr (BIASED) {
-            return indexed ? cdf_find(g, beg, (int)d, x, T) : (int)search_upper(P, d, its_target(x, T));
+            if (indexed) return FAR ? cdf_find_far(g, beg, (int)d, x, T) : cdf_find(g, beg, (int)d, x, T);
+            return (int)search_upper(P, d, its_target(x, T));
         } else {
             return kth_not_excluded(mulhi(x, (uint32_t)(d - nZ)), zs, nZ);
         }
@@ -156,7 +158,7 @@ __device__ __forceinline__ void stream_bases(DevGraph &g, const LevelArgs &a, in
 // reads the adjacency of its own partition (LevelArgs::part_col/part_w) and
 // items of partitions not sampled this round are skipped.
 template <typename I, int BIAS, bool STREAM = false>
-__global__ void __launch_bounds__(EXPAND_THREADS)
+__global__ void __launch_bounds__(EXPAND_THREADS, STREAM ? 4 : 1)
 k_expand_warp(DevGraph g0, LevelArgs a) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
     constexpr int NW = EXPAND_THREADS / 32;
@@ -220,7 +222,8 @@ k_expand_warp(DevGraph g0, LevelArgs a) {
             if (d > N) {
                 scanned = BIASED && !(g.cdf && g.cdf_bias == BIAS);
                 const DrawCtx dc{a.k0, a.k1, p, (uint32_t)s, (uint32_t)l};
-                sel = select_warp<I, BIAS>(g, beg, d, N, dc, P, zb, zs, lane, WBUF);
+                sel = select_warp<I, BIAS, STREAM>(g, beg, d, N, dc, P, zb, zs, lane, WBUF,
+                                                   STREAM && a.row_total ? __ldg(a.row_total + v) : -1.f);
                 if (sel == -2) {   // cached hub that needs a rebuild: the CTA path redoes it
                     // (only with a prefix cache, which streaming graphs do not have)
                     my_items--;
@@ -933,6 +936,17 @@ __global__ void k_cdf_build_big(DevGraph g, float *cdf, const int32_t *verts, in
         float *gcar = tsum + (d >> 5) + 1;
         auto wfn = [&](int64_t i) { return edge_bias<I, BIAS>(g, beg + i); };
         cta_canon_prefix(wfn, d, cdf + beg, tsum, gcar, nullptr);
+    }
+}
+
+// Row totals of vertices [v0, v1): the last prefix entry (cdf indexed by global
+// edge), 0 for a row without edges.
+template <typename I>
+__global__ void k_row_total(DevGraph g, const float *cdf, float *total, int64_t v0, int64_t v1) {
+    for (int64_t v = v0 + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < v1;
+         v += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t beg = row_begin<I>(g, v), end = row_begin<I>(g, v + 1);
+        total[v] = end > beg ? cdf[end - 1] : 0.f;
     }
 }
 

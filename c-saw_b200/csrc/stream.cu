@@ -175,6 +175,7 @@ struct csaw_stream_graph_s {
     // prefix of every row in page-locked host memory, streamed in place of the
     // weights, and its two index levels resident on the device.
     float *h_cdf[4] = {};
+    float *d_tot[4] = {};             // per vertex: its row's prefix total (null: read from the prefix)
     float *d_idx[4] = {};             // cdf1 [(E + 31) / 32], then cdf2 [(E + 1023) / 1024]
     StreamCounters *hctr = nullptr;
     int64_t loads = 0, hits = 0, bytes_h2d = 0, launches = 0;
@@ -530,6 +531,7 @@ int run_stream(csaw_stream_graph_s *g, const csaw_params *p, const int fan[], co
             if (cached) {
                 a.cdf1_all = g->d_idx[BIAS];
                 a.cdf2_all = g->d_idx[BIAS] + ((g->E + 31) >> 5);
+                a.row_total = g->d_tot[BIAS];
                 a.host_w = g->reg_w ? g->h_w : nullptr;   // page-locked in place: device-readable
             }
             a.out_v = qv(U, 0);
@@ -698,6 +700,7 @@ extern "C" int csaw_stream_graph_destroy(csaw_stream_graph g) {
     for (int b = 0; b < 4; ++b) {
         if (g->h_cdf[b]) cudaFreeHost(g->h_cdf[b]);
         if (g->d_idx[b]) cudaFree(g->d_idx[b]);
+        if (g->d_tot[b]) cudaFree(g->d_tot[b]);
     }
     cudaGetLastError();
     delete g;
@@ -728,7 +731,7 @@ int build_stream_cdf(csaw_stream_graph_s *g) {
         cudaFree(stage_cdf);
         cudaGetLastError();
     };
-    if (cudaHostAlloc((void **)&h, sizeof(float) * (size_t)std::max<int64_t>(E, 1), cudaHostAllocDefault) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&h, sizeof(float) * (size_t)((E + 8) & ~7ll), cudaHostAllocDefault) != cudaSuccess) {   // whole sectors
         cudaGetLastError();
         return csaw_host_fail(CSAW_ERR_NOMEM, "page-locked prefix cache allocation failed");
     }
@@ -751,6 +754,14 @@ int build_stream_cdf(csaw_stream_graph_s *g) {
         }
     };
     ck(cudaMemsetAsync(idx, 0, sizeof(float) * (size_t)(n1 + n2), st), "index clear");
+    // row totals on the device: a draw then reads none over the link (4 V
+    // bytes; without the memory for them the total is read from the prefix)
+    float *tot = nullptr;
+    if (cudaMalloc((void **)&tot, sizeof(float) * (size_t)g->V) != cudaSuccess) {
+        cudaGetLastError();
+        tot = nullptr;
+    }
+    if (tot) ck(cudaMemsetAsync(tot, 0, sizeof(float) * (size_t)g->V, st), "totals clear");
     for (int q = 0; q < g->npart && !rc; ++q) {
         const int64_t e0 = g->pbeg[q], e1 = g->pbeg[q + 1], ne = e1 - e0;
         if (ne == 0) continue;
@@ -768,6 +779,10 @@ int build_stream_cdf(csaw_stream_graph_s *g) {
         k_cdf_build<I, BIAS><<<g->sm_count * 8, 256, 0, st>>>(dg, stage_cdf - e0, INT64_MAX, v0, v1);
         k_cdf_index_range<<<g->sm_count * 2, 256, 0, st>>>(stage_cdf - e0, e0, e1, idx, idx + n1);
         g->launches += 2;
+        if (tot) {
+            k_row_total<I><<<g->sm_count * 2, 256, 0, st>>>(dg, stage_cdf - e0, tot, v0, v1);
+            g->launches++;
+        }
         ck(cudaGetLastError(), "prefix build launch");
         ck(cudaMemcpyAsync(h + e0, stage_cdf, sizeof(float) * ne, cudaMemcpyDeviceToHost, st), "prefix copy");
         ck(cudaStreamSynchronize(st), "prefix build");   // the staging buffers are reused
@@ -775,10 +790,12 @@ int build_stream_cdf(csaw_stream_graph_s *g) {
     cleanup();
     if (rc) {
         cudaFree(idx);
+        cudaFree(tot);
         cudaFreeHost(h);
         return rc;
     }
     g->h_cdf[BIAS] = h;
+    g->d_tot[BIAS] = tot;
     g->d_idx[BIAS] = idx;
     void *dp = nullptr;
     if (cudaHostGetDevicePointer(&dp, h, 0) == cudaSuccess) g->dv_cdf[BIAS] = (const float *)dp;

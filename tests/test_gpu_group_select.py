@@ -75,3 +75,25 @@ def test_group_pass_equals_oracle(csaw, rows_graph, rowptr64, bias, n_slots):
     ref = oracle.run(g.rowptr, g.col, g.weight, seeds, 0, bias, n, 1, 2, fan, seed=seed, n_threads=8)
     a, b = sort_edges(*out), sort_edges(*ref)
     assert a.shape == b.shape and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("rowptr64", [False, True])
+@pytest.mark.parametrize("bias", [1, 2])
+def test_rows_read_in_place_equal_oracle(csaw, rows_graph, rowptr64, bias):
+    """The same rows from a streaming graph: the first job finds no partition on
+    the device and reads the page-locked host prefix sector by sector, the
+    second reads the partitions' device copies."""
+    import torch
+    g, hubs = rows_graph
+    G = csaw.StreamGraph(g, partition_bits=6, slot_budget_bytes=16 * int(g.rowptr[hubs]), rowptr64=rowptr64)
+    G.cache(bias)
+    n = hubs * 5 + 3
+    seeds = (np.arange(n) % hubs).astype(np.int32)
+    for mode, fan, depth in ((0, [7, 2], 2), (1, None, 12), (0, [7, 2], 2), (1, None, 12)):
+        p = csaw.make_params(mode, bias, n, 1, (fan or [1])[0], depth, fan, 77)
+        out = [x.cpu().numpy() for x in G.sample(p, torch.from_numpy(seeds).cuda())]
+        ref = oracle.run(g.rowptr, g.col, g.weight, seeds, mode, bias, n, 1, depth, fan, seed=77, n_threads=8)
+        a, b = sort_edges(*out), sort_edges(*ref)
+        assert a.shape == b.shape and np.array_equal(a, b), (mode, depth)
+    assert G.info()["items_read_in_place"] > 0
+    G.close()
