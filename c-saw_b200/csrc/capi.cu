@@ -71,7 +71,9 @@ struct Counters {
     uint32_t n_refill;
     uint32_t n_thread;
     int err;
+    uint32_t ticket;      // CTAs of a counting kernel that have ended (CounterOut)
 };
+static_assert(sizeof(Counters) % sizeof(uint32_t) == 0, "read back word by word");
 
 struct DevBuf {
     void *p = nullptr;
@@ -132,6 +134,9 @@ struct JobCtx {
         pctr,   // per-level counters and barrier words of a persistent job
         tsel;   // thread-per-item list
     Counters *ctr = nullptr, *hctr = nullptr;
+    bool ctr_zero = false;           // ctr is zero once the work queued so far is done
+    bool self_count = false;         // a job's only kernel may read its counters back itself ...
+    bool self_counted = false;       // ... and does
     cudaStream_t stream = nullptr;   // owned (batch jobs); job 0 uses the caller's
     cudaEvent_t done = nullptr;
     cudaStream_t side = nullptr;     // CTA-granularity pass, concurrent with the warp pass
@@ -294,12 +299,30 @@ void drain_profile(csaw_graph_s *g) {
     g->pending.clear();
 }
 
+// The occupancy-filled grid of a kernel.  The query costs a microsecond or
+// two a kernel and a job asks for several, so each thread keeps the answers
+// (they depend on the kernel and the device type alone).
 template <typename K>
 int grid_for(K kernel, int threads, size_t dyn_smem, int sm_count) {
+    thread_local std::map<std::array<size_t, 3>, int> known;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    const std::array<size_t, 3> key{(size_t)(const void *)kernel, dyn_smem, (size_t)threads * 1024 + (size_t)dev};
+    const auto it = known.find(key);
+    if (it != known.end()) return it->second * sm_count;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, dyn_smem);
     if (per_sm < 1) per_sm = 1;
+    if (known.size() >= 256) known.clear();
+    known[key] = per_sm;
     return per_sm * sm_count;
+}
+
+// The counter block for a job's only kernel to read back, or nothing.
+CounterOut counter_out(JobCtx *c) {
+    if (!c->self_count) return CounterOut{};
+    c->self_counted = true;
+    return CounterOut{(uint32_t *)c->ctr, (uint32_t *)c->hctr, (int)(sizeof(Counters) / 4), &c->ctr->ticket};
 }
 
 // Per-edge neighbor records, built once per graph on first batched use
@@ -568,6 +591,7 @@ int run_tree(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int fan[], 
     t.F = p->frontier_size;
     t.base = (int)p->sample_base;
     const DevGraph dg = dev_view(g, p->schedule, BIAS);
+    t.done = counter_out(c);
     LaunchScope ls(g, KK_TREE, st);
     k_tree<I, BIAS><<<(unsigned)grid, threads, m.bytes, st>>>(dg, t);
     CK(cudaGetLastError());
@@ -978,6 +1002,7 @@ int run_walk_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
     a.err = &c->ctr->err;
     a.k0 = (uint32_t)p->seed;
     a.k1 = (uint32_t)(p->seed >> 32);
+    a.done = counter_out(c);
     if (BIAS == CSAW_BIAS_UNBIASED) {
         // many unbiased walks are bound by their scattered sectors: where the
         // 16-byte records are larger than L2 and the row offsets are not, the
@@ -1046,6 +1071,7 @@ int run_mdrw_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
     a.err = &c->ctr->err;
     a.k0 = (uint32_t)p->seed;
     a.k1 = (uint32_t)(p->seed >> 32);
+    a.done = counter_out(c);
     if (a.F <= 32) {
         const int gmax = grid_for(k_mdrw_warp<I, BIAS>, WALK_THREADS, 0, g->sm_count);
         const int grid = std::max(1, std::min((p->n_samples + WALK_THREADS / 32 - 1) / (WALK_THREADS / 32), gmax));
@@ -1165,7 +1191,16 @@ int enqueue_job(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t 
     if (cap < 0) return fail(CSAW_ERR_INVALID, "capacity < 0");
     if (cap > 0 && (!src || !dst)) return fail(CSAW_ERR_INVALID, "out_src/out_dst are NULL");
     if (p->n_samples > 0 && !seeds) return fail(CSAW_ERR_INVALID, "seeds is NULL");
-    if (reset) CK(cudaMemsetAsync(c->ctr, 0, sizeof(Counters), st));
+    // Jobs of one kernel (sample trees, walks, MDRW) read their counters back
+    // themselves: no clearing before and no copy behind them.  Not while a
+    // graph is captured (its replays must not depend on what ran before) nor
+    // for host-buffer jobs, which post the running count behind the kernel.
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const bool eager = cudaStreamIsCapturing(st, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+    if (reset && !(eager && c->ctr_zero)) CK(cudaMemsetAsync(c->ctr, 0, sizeof(Counters), st));
+    c->ctr_zero = false;
+    c->self_count = reset && eager && !c->posting;
+    c->self_counted = false;
     OutArgs o{src, dst, smp, dep, &c->ctr->out_count, cap};
     c->trial_arm = -1;
     const bool timed = g->trial && p->schedule == CSAW_SCHED_LEARNED && p->mode == CSAW_MODE_NEIGHBOR &&
@@ -1184,7 +1219,8 @@ int enqueue_job(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t 
         CK(cudaEventRecord(c->t1, st));
         c->trial_arm = g->trial_arm;
     }
-    CK(cudaMemcpyAsync(c->hctr, c->ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
+    if (c->self_counted) c->ctr_zero = true;
+    else CK(cudaMemcpyAsync(c->hctr, c->ctr, sizeof(Counters), cudaMemcpyDeviceToHost, st));
     return 0;
 }
 

@@ -66,6 +66,15 @@ struct SelEntry {
 
 struct SchedArgs;
 
+// Where a job's only kernel leaves its counter block: page-locked host words
+// (null: nowhere), the device words cleared behind it; ticket is one of them.
+struct CounterOut {
+    uint32_t *dev;
+    uint32_t *host;
+    int words;
+    uint32_t *ticket;
+};
+
 // One level of neighbor sampling: input queue -> output edges + next queue.
 struct LevelArgs {
     const int32_t *in_v;
@@ -165,6 +174,7 @@ struct WalkArgs {
     unsigned long long *items;
     int *err;
     uint32_t k0, k1;
+    CounterOut done;
 };
 
 enum : int { ERR_SEED_RANGE = 1, ERR_UPDATE_RANGE = 2, ERR_SCRATCH = 4, ERR_COPY_WAIT = 8, ERR_BARRIER = 16 };

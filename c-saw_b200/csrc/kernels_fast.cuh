@@ -1214,6 +1214,7 @@ k_walk_fast(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[2], bytes + steps * (obytes + rec) + 128ull * (rounds / 5));   // 32 probes a round
         atomicAdd(&a.items[2], steps);
     }
+    counters_out(a.done);
 }
 
 // Walks with one thread per walk, for many walks: unbiased steps take one
@@ -1364,6 +1365,7 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[8], tot * per + 4 * pr);   // + prefix probes (biased)
         atomicAdd(&a.items[8], tot);
     }
+    counters_out(a.done);
 }
 
 // MDRW with a frontier of at most 32 vertices: one warp per sample, slot i on
@@ -1460,6 +1462,7 @@ k_mdrw_warp(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[3], visits * 2ull * sizeof(I) + steps * (4ull + 4ull * (2 + (a.o_smp != nullptr) + (a.o_dep != nullptr))));
         atomicAdd(&a.items[3], steps);
     }
+    counters_out(a.done);
 }
 
 template <typename I>

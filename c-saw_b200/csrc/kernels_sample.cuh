@@ -750,6 +750,7 @@ k_walk_thread(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[8], tot * per);
         atomicAdd(&a.items[8], tot);
     }
+    counters_out(a.done);
 }
 
 // Biased walks: one warp per walk; per step the warp builds the canonical
@@ -831,6 +832,7 @@ k_walk_warp(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[2], bytes);
         atomicAdd(&a.items[2], steps);
     }
+    counters_out(a.done);
 }
 
 // ------------------------------------------------------------- MDRW
@@ -906,6 +908,7 @@ __global__ void k_mdrw(DevGraph g, WalkArgs a) {
         atomicAdd(&a.bytes[3], bytes);
         atomicAdd(&a.items[3], steps);
     }
+    counters_out(a.done);
 }
 
 // -------------------------------------------------------------- CDF cache

@@ -44,6 +44,7 @@ struct TreeArgs {
     int n_samples, F, base, per_chunk, n_chunks;
     uint32_t qoff[TREE_MAX_LEVELS + 1];    // first queue entry of level l; [D] the chunk's total
     uint32_t wmax;                         // entries of the widest level
+    CounterOut done;
 };
 
 // Byte offsets of the dynamic shared memory of k_tree for nw warps.
@@ -414,6 +415,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
         atomicAdd(&a.bytes[kind], s_bytes[tid]);
         atomicAdd(&a.items[kind], (unsigned long long)s_items[tid]);
     }
+    counters_out(t.done);
 }
 
 }  // namespace csaw
