@@ -1828,6 +1828,7 @@ extern "C" int csaw_sample_batch(csaw_graph g, csaw_job *jobs, int n_jobs, void 
                 ctx[i] = g->jobs[(size_t)i + 1];
                 jobs[i].status = 0;
             }
+            for (JobCtx *c : ctx) c->ctr_zero = false;   // the replay leaves its counts behind
             CK(cudaGraphLaunch(it->second, st));
             g->launches += g->graph_kernels[key];
             launched = true;
