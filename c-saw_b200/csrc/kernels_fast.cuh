@@ -429,8 +429,12 @@ __device__ __forceinline__ void emit_edge(const DevGraph &g, const LevelArgs &a,
 template <typename I, int BIAS>
 __device__ __forceinline__ void coop_body(const DevGraph &g, const LevelArgs &a) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
-    const int lane = threadIdx.x & 31;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    constexpr int NW = FAST_THREADS / 32;
+    // per reservation (output, next queue, warp, thread, group and hub list,
+    // four CTA lists): each warp's count, then its range's start
+    __shared__ uint32_t s_cnt[9][NW], s_at[9][NW];
+    __shared__ unsigned long long s_ob[NW];
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
     const uint32_t n = __ldcg(a.n_in);
     const int N = a.N;
@@ -442,8 +446,8 @@ __device__ __forceinline__ void coop_body(const DevGraph &g, const LevelArgs &a)
     uint32_t bs = (n + nw - 1) / nw;
     bs = bs < 1 ? 1 : (bs > 32 ? 32 : bs);
     unsigned long long my_bytes = 0, my_items = 0;
-    for (uint32_t base = gw * bs; base < n; base += nw * bs) {
-        const uint32_t it = base + lane;
+    for (uint32_t cta = blockIdx.x * NW * bs; cta < n; cta += nw * bs) {
+        const uint32_t it = cta + wib * bs + lane;
         const bool valid = lane < (int)bs && it < n;
         int32_t v = 0, s = 0;
         uint32_t p = 0;
@@ -491,9 +495,10 @@ __device__ __forceinline__ void coop_body(const DevGraph &g, const LevelArgs &a)
         const int excl = incl - k;
         const int K = __shfl_sync(FULL, incl, 31);
         // Items that need draws go to one list each, with their reserved
-        // slots.  Lane 0 reserves the batch's output and queue slots and its
-        // range in every list at once: the atomics are independent, so their
-        // round trips overlap instead of following one another.
+        // slots.  The CTA reserves its warps' output and queue slots and their
+        // ranges in every list together, a counter a thread: every warp of the
+        // GPU adds to the same few words, and an add per warp and counter was
+        // half of the pass's time.
         const bool to_sel = drawn && !heavy && !hub && !pair && !thr;
         const unsigned sm = __ballot_sync(FULL, to_sel);
         const unsigned tm = __ballot_sync(FULL, thr);
@@ -502,43 +507,62 @@ __device__ __forceinline__ void coop_body(const DevGraph &g, const LevelArgs &a)
         unsigned cm[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) cm[c] = __ballot_sync(FULL, heavy && cls == 2 + c);
-        unsigned long long ob = 0;
-        uint32_t qb = 0, ps = 0, pt = 0, pp = 0, ph = 0, pc[4] = {0u, 0u, 0u, 0u};
         if (lane == 0) {
-            if (K) {
-                ob = atomicAdd(a.o_count, (unsigned long long)K);
-                if (a.push) qb = atomicAdd(a.n_out, (uint32_t)K);
-            }
-            if (sm) ps = atomicAdd(a.n_sel, (uint32_t)__popc(sm));
-            if (tm) pt = atomicAdd(a.n_thread, (uint32_t)__popc(tm));
-            if (pbm) pp = atomicAdd(a.n_pair, (uint32_t)__popc(pbm));
-            if (hbm) ph = atomicAdd(a.n_hub, (uint32_t)__popc(hbm));
+            s_cnt[0][wib] = (uint32_t)K;
+            s_cnt[1][wib] = (uint32_t)__popc(sm);
+            s_cnt[2][wib] = (uint32_t)__popc(tm);
+            s_cnt[3][wib] = (uint32_t)__popc(pbm);
+            s_cnt[4][wib] = (uint32_t)__popc(hbm);
 #pragma unroll
-            for (int c = 0; c < 4; ++c)
-                if (cm[c]) pc[c] = atomicAdd(&a.n_cta[c], (uint32_t)__popc(cm[c]));
+            for (int c = 0; c < 4; ++c) s_cnt[5 + c][wib] = (uint32_t)__popc(cm[c]);
         }
-        ob = __shfl_sync(FULL, ob, 0);
-        qb = __shfl_sync(FULL, qb, 0);
+        __syncthreads();
+        if (threadIdx.x < 10) {   // 0: the output; 1..8: the lists; 9: the next queue
+            const int k9 = threadIdx.x == 9 ? 0 : threadIdx.x;
+            uint32_t tot = 0;
+#pragma unroll
+            for (int w = 0; w < NW; ++w) tot += s_cnt[k9][w];
+            if (threadIdx.x == 0) {
+                unsigned long long at = tot ? atomicAdd(a.o_count, (unsigned long long)tot) : 0ull;
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    s_ob[w] = at;
+                    at += s_cnt[0][w];
+                }
+            } else {
+                uint32_t *ctr = threadIdx.x == 1   ? a.n_sel
+                                : threadIdx.x == 2 ? a.n_thread
+                                : threadIdx.x == 3 ? a.n_pair
+                                : threadIdx.x == 4 ? a.n_hub
+                                : threadIdx.x == 9 ? a.n_out
+                                                   : a.n_cta + (threadIdx.x - 5);
+                uint32_t at = tot && (threadIdx.x != 9 || a.push) ? atomicAdd(ctr, tot) : 0u;
+                uint32_t *to = threadIdx.x == 9 ? s_at[0] : s_at[threadIdx.x];
+#pragma unroll
+                for (int w = 0; w < NW; ++w) {
+                    to[w] = at;
+                    at += s_cnt[k9][w];
+                }
+            }
+        }
+        __syncthreads();
+        const unsigned long long ob = s_ob[wib];
+        const uint32_t qb = s_at[0][wib];
         const unsigned below = (1u << lane) - 1u;
         const SelEntry en{it, qb + (uint32_t)excl, ob + excl, v, s, p, (int32_t)d, (long long)beg, cls, 0};
         {
-            const uint32_t pos_s = __shfl_sync(FULL, ps, 0), pos_t = __shfl_sync(FULL, pt, 0);
-            const uint32_t pos_p = __shfl_sync(FULL, pp, 0), pos_h = __shfl_sync(FULL, ph, 0);
-            uint32_t pos_c[4];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) pos_c[c] = __shfl_sync(FULL, pc[c], 0);
             if (to_sel) {
-                a.sel_list[pos_s + __popc(sm & below)] = en;
+                a.sel_list[s_at[1][wib] + __popc(sm & below)] = en;
             } else if (thr) {
-                a.thread_list[pos_t + __popc(tm & below)] = en;
+                a.thread_list[s_at[2][wib] + __popc(tm & below)] = en;
             } else if (pair) {
-                a.pair_list[pos_p + __popc(pbm & below)] = en;
+                a.pair_list[s_at[3][wib] + __popc(pbm & below)] = en;
             } else if (hub) {
-                a.hub_list[pos_h + __popc(hbm & below)] = en;
+                a.hub_list[s_at[4][wib] + __popc(hbm & below)] = en;
             } else if (heavy) {
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
-                    if (cls == 2 + c) a.cta_list[c][pos_c[c] + __popc(cm[c] & below)] = en;
+                    if (cls == 2 + c) a.cta_list[c][s_at[5 + c][wib] + __popc(cm[c] & below)] = en;
             }
         }
         if (valid) {
