@@ -225,9 +225,16 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
             if (tid == T - 32) s_ob = total ? atomicAdd(a.o_count, (unsigned long long)total) : 0ull;
             if (n > 32) __syncthreads();   // every item's offset
             const uint32_t ndraw = s_ndraw, ngroup = s_ngroup;
-            bool met = false;   // the warp has passed the barrier after which s_ob is there
+            // The barrier after which s_ob is there, passed by every thread
+            // once a level.  It follows loads under `if (act)`, after which
+            // the source alone does not say that the warp has converged, so it
+            // is the form that does not ask for it (bar.sync does).
+            bool met = false;   // the same in all lanes of a warp
             auto meet = [&]() {
-                if (!met) asm volatile("bar.sync 1, %0;" ::"r"(T) : "memory");
+                if (!met) {
+                    __syncwarp();
+                    asm volatile("barrier.sync 1, %0;" ::"r"(T) : "memory");
+                }
                 met = true;
             };
             // edge j of queue item i, its neighbor at offset off of the row:
