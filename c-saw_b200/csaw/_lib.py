@@ -38,6 +38,7 @@ OPT_RETRY_SMEM = 6
 OPT_PERSISTENT = 7
 OPT_THREAD_SELECT = 8
 OPT_INCR_REBUILD = 9
+OPT_TREE = 10
 STREAM_OPT_READ_IN_PLACE = 1
 MLP_NPARAM, MLP_NORM = 1575, 18
 

@@ -180,6 +180,7 @@ struct csaw_graph_s {
     int retry_smem = 0;           // CSAW_OPT_RETRY_SMEM (bytes)
     bool persistent = false;      // CSAW_OPT_PERSISTENT
     int thread_sel = 1;           // CSAW_OPT_THREAD_SELECT: 0 off, 1 degree rule, 2 every d <= 32 item
+    int tree = 1;                 // CSAW_OPT_TREE: 0 never, 1 by size, 2 wherever a sample fits
     uint32_t class_mask = 0x7f;   // classes the trained model picks (bit c)
     int32_t *big_verts = nullptr; // vertices above CDF_BIG (the cache builds them one CTA each)
     int64_t n_big = 0;
@@ -515,9 +516,9 @@ bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], Tr
     const bool plain = p->schedule == CSAW_SCHED_PLAIN;
     if (BIASED && (plain || g->cdf_off)) return false;
     if ((p->flags & CSAW_PARAM_DEDUP) && D > 1) return false;
-    if (D > TREE_MAX_LEVELS || g->E == 0) return false;
+    if (D > TREE_MAX_LEVELS || g->E == 0 || g->tree == 0) return false;
     // launch-shape options keep the launches they shape
-    if (!plain && (g->persistent || g->grid_pct != 100 || !g->pair || g->thread_sel == 2)) return false;
+    if (g->tree == 1 && !plain && (g->persistent || g->grid_pct != 100 || !g->pair || g->thread_sel == 2)) return false;
     if (p->schedule == CSAW_SCHED_LEARNED && BIASED) {   // only where the degree rule routes
         const bool model = g->trained && (g->class_mask & 0x7cu) && !g->mlp_lost && !(g->trial && g->trial_arm == 0);
         if (g->recording || model) return false;
@@ -533,7 +534,7 @@ bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], Tr
     }
     off[D] = (uint32_t)tot;
     if (tot > TREE_MAX_ITEMS) return false;
-    if (tot * S > (double)TREE_JOB_ITEMS) return false;
+    if (g->tree == 1 && tot * S > (double)TREE_JOB_ITEMS) return false;
     // the widest CTAs (512 threads down to 128) whose chunks of one sample
     // are all resident at once, 1024 threads an SM; more samples than that
     // share chunks.  Us a call: 64 seeds [25,10] 69 at 512 threads, 79 at
@@ -1941,6 +1942,11 @@ extern "C" int csaw_graph_set_option(csaw_graph g, int option, int64_t value) {
         case CSAW_OPT_THREAD_SELECT:
             if (value < 0 || value > 2) return fail(CSAW_ERR_INVALID, "thread select: 0, 1 or 2");
             g->thread_sel = (int)value;
+            ++g_alloc_epoch;   // launch structure is baked into cached graphs
+            return 0;
+        case CSAW_OPT_TREE:
+            if (value < 0 || value > 2) return fail(CSAW_ERR_INVALID, "tree: 0, 1 or 2");
+            g->tree = (int)value;
             ++g_alloc_epoch;   // launch structure is baked into cached graphs
             return 0;
         case CSAW_OPT_PERSISTENT:

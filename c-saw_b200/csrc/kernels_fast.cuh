@@ -1385,7 +1385,9 @@ k_walk_thread_fast(DevGraph g, WalkArgs a) {
         pr += __shfl_xor_sync(FULL, pr, off);
     }
     if (lane == 0) {
-        unsigned long long per = 4 + sizeof(I) + 4 + 4ull * (2 + (a.o_smp != nullptr) + (a.o_dep != nullptr));
+        // the column and a record's row range, or (by_col) two row offsets
+        unsigned long long per = 4 + sizeof(I) + (a.by_col ? sizeof(I) : 4) +
+                                 4ull * (2 + (a.o_smp != nullptr) + (a.o_dep != nullptr));
         atomicAdd(&a.bytes[8], tot * per + 4 * pr);   // + prefix probes (biased)
         atomicAdd(&a.items[8], tot);
     }

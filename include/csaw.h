@@ -255,7 +255,15 @@ enum {
      * its prefix incrementally from per-tile summaries built with the cache
      * (8 bytes per 32 edges of the hub rows, E/32 + V + 1 slots); 0: every
      * rebuild rescans the whole row.  Never changes the output. */
-    CSAW_OPT_INCR_REBUILD = 9
+    CSAW_OPT_INCR_REBUILD = 9,
+    /* Whole sample trees in one launch (neighbor jobs without dedup of up to
+     * 8 hops, unbiased or with the degree rule over a cached prefix, the
+     * plain schedule's unbiased jobs among them).  1 (default): small and
+     * middle jobs, by size, unless one of the launch-shape options above is
+     * set; 0: never, a launch or more per level; 2: every job whose samples
+     * fit one CTA's shared memory (4096 frontier items a sample).  Never
+     * changes the output. */
+    CSAW_OPT_TREE = 10
 };
 int csaw_graph_set_option(csaw_graph g, int option, int64_t value);
 
