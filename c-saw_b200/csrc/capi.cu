@@ -157,6 +157,26 @@ struct JobCtx {
 
 }  // namespace
 
+// Degrees of a sample of vertices, by fan-out N: the share above N, and the
+// mean of min(degree, N).
+struct DegreeShare {
+    float above[MAX_FANOUT + 1] = {}, fill[MAX_FANOUT + 1] = {};
+    double weight = 0;
+    void add(int64_t d, double w) {
+        for (int N = 0; N <= MAX_FANOUT; ++N) {
+            above[N] += d > N ? (float)w : 0.f;
+            fill[N] += (float)(w * (double)std::min<int64_t>(d, N));
+        }
+        weight += w;
+    }
+    void finish() {
+        for (int N = 0; N <= MAX_FANOUT && weight > 0; ++N) {
+            above[N] /= (float)weight;
+            fill[N] /= (float)weight;
+        }
+    }
+};
+
 struct csaw_graph_s {
     int device = 0, sm_count = 148;
     int64_t l2_bytes = 126ll << 20;
@@ -180,6 +200,7 @@ struct csaw_graph_s {
     int retry_smem = 0;           // CSAW_OPT_RETRY_SMEM (bytes)
     bool persistent = false;      // CSAW_OPT_PERSISTENT
     int thread_sel = 1;           // CSAW_OPT_THREAD_SELECT: 0 off, 1 degree rule, 2 every d <= 32 item
+    DegreeShare roots, children[2];   // of seeds drawn uniformly; of neighbors (and weighted by their degree)
     int tree = 1;                 // CSAW_OPT_TREE: 0 never, 1 by size, 2 wherever a sample fits
     uint32_t class_mask = 0x7f;   // classes the trained model picks (bit c)
     int32_t *big_verts = nullptr; // vertices above CDF_BIG (the cache builds them one CTA each)
@@ -497,17 +518,30 @@ void post_count(csaw_graph_s *g, JobCtx *c, cudaStream_t st) {
 }
 
 // Neighbor jobs whose sample trees run whole in one launch (k_tree): those
-// whose frontier levels hold at most this many items, counted by their bound
-// (FrontierSize x the fan-outs).  Below it the per-level launches are most of
-// a job's time; above it a chunk's levels, one after another on one SM, cost
-// more than launches that spread every level over the GPU.  Per-level passes
-// and one launch, us a call on a B200: 64 seeds [25,10] 123 and 69, 1024 148
-// and 78, 8192 (213 K items by the bound) 215 and 176, 16384 (426 K) 243 and
-// 265; 1024 seeds [15,10,5] (170 K) 245 and 129, 4096 (680 K) 329 and 500
-// (R-MAT 22, edge weights); F4 [20,20,20] on the power-law graph, 64 samples
-// (108 K) 128 and 92, 1024 (1.7 M) 173 and 239; unbiased [15,10], 16384 seeds
-// (262 K) 181 and 164; plain unbiased F4 [10,10], 8000 (352 K) 198 and 201.
+// whose frontier levels hold at most TREE_JOB_ITEMS items, counted by their
+// bound (FrontierSize x the fan-outs).  Below it the per-level launches are
+// most of a job's time; above it a chunk's levels, one after another on one
+// SM, cost more than launches that spread every level over the GPU.
+// Per-level passes and one launch, us a call on a B200: 64 seeds [25,10] 112
+// and 57, 1024 131 and 77, 8192 (213 K items by the bound) 198 and 176, 16384
+// (426 K) 238 and 296; 1024 seeds [15,10,5] (170 K) 230 and 137, 4096 (680 K)
+// 314 and 579 (R-MAT 22, edge weights); F4 [20,20,20] on the power-law graph,
+// degree bias, 64 samples (108 K) 119 and 85, 1024 (1.7 M) 151 and 272.
+// Unbiased jobs gain for longer ([15,10] on R-MAT 22, 65,536 seeds, 1 M items:
+// 375 and 283); the line is the biased jobs'.
 constexpr int64_t TREE_JOB_ITEMS = 1 << 18;
+// ... and whose chunks keep a warp busy for no more than this many rounds, a
+// round being one item that needs draws, or 32 / N of them for N <= 16.  A
+// chunk has one SM, so a wide tree of few roots waits for its rounds there
+// while the rest of the GPU idles.  The rounds are those expected from the
+// graph's degrees (a power-law graph takes most rows whole: no draws).
+// Per-level passes and one launch, us, edge weights: [32,32,32], 16 seeds,
+// R-MAT 22 (52 rounds) 158 and 334; F4 [20,20,20], 64 samples, R-MAT 22 (21)
+// 206 and 216, power-law graph (0.2) 113 and 68; F4 [10,10,10], 512 samples,
+// R-MAT 22 (17) 254 and 199; F4 [31,32], 1024 samples, heavy-tailed R-MAT 20
+// (24) 292 and 411.
+constexpr double TREE_CHUNK_ROUNDS = 20;
+constexpr int64_t DEGREE_SAMPLE = 1 << 14;   // vertices and edges a graph's DegreeShare is made of
 
 template <typename I, int BIAS>
 bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], TreeArgs *t, int *threads) {
@@ -523,7 +557,7 @@ bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], Tr
         const bool model = g->trained && (g->class_mask & 0x7cu) && !g->mlp_lost && !(g->trial && g->trial_arm == 0);
         if (g->recording || model) return false;
     }
-    double w = F, tot = 0;
+    double w = 1, tot = 0;   // items of one root's tree, by level
     uint32_t off[TREE_MAX_LEVELS + 1], wmax = 0;
     for (int l = 0; l < D; ++l) {
         if (w > TREE_MAX_ITEMS) return false;
@@ -533,20 +567,32 @@ bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], Tr
         w *= fan[l];
     }
     off[D] = (uint32_t)tot;
-    if (tot > TREE_MAX_ITEMS) return false;
-    if (g->tree == 1 && tot * S > (double)TREE_JOB_ITEMS) return false;
-    // the widest CTAs (512 threads down to 128) whose chunks of one sample
-    // are all resident at once, 1024 threads an SM; more samples than that
-    // share chunks.  Us a call: 64 seeds [25,10] 69 at 512 threads, 79 at
-    // 128; 1024 seeds 79 at 128, 95 at 256 (two waves); 3001 unbiased [15,10]
-    // seeds 71 in chunks of 2 or 3, 80 in chunks of one
-    const int64_t room = 1024ll * g->sm_count;
+    if (tot * F > TREE_MAX_ITEMS || (double)S * F > INT32_MAX) return false;
+    if (g->tree == 1 && tot * F * S > (double)TREE_JOB_ITEMS) return false;
+    // a chunk is a run of roots: trees of one sample do not meet either.  The
+    // widest CTAs (512 threads down to 128) whose chunks of one root are all
+    // resident at once, 1024 threads an SM; more roots than that share chunks.
+    // Us a call: 64 seeds [25,10] 69 at 512 threads, 79 at 128; 1024 seeds 79
+    // at 128, 95 at 256 (two waves); 3001 unbiased [15,10] seeds 71 in chunks
+    // of 2 or 3, 80 in chunks of one.  (Chunks of whole samples: one unbiased
+    // sample F64 [16,2,2] on R-MAT 20 194 us, the per-level passes 88, now 44.)
+    const int64_t room = 1024ll * g->sm_count, roots = (int64_t)S * F;
     int T = 512;
-    while (T > 128 && (int64_t)S * T > room) T >>= 1;
-    int C = (int)std::min<int64_t>(((int64_t)S * T + room - 1) / room, TREE_MAX_ITEMS);
-    C = std::min(C, (int)(TREE_MAX_ITEMS / tot));
-    t->per_chunk = C;
-    t->n_chunks = (S + C - 1) / C;
+    while (T > 128 && roots * T > room) T >>= 1;
+    int64_t C = std::min<int64_t>((roots * T + room - 1) / room, (int64_t)(TREE_MAX_ITEMS / tot));
+    t->per_chunk = (int)C;
+    t->n_chunks = (int)((roots + C - 1) / C);
+    if (g->tree == 1) {
+        const DegreeShare &child = g->children[BIAS == CSAW_BIAS_DEGREE];
+        double items = (double)std::min(C, roots), rounds = 0;
+        for (int l = 0; l < D; ++l) {
+            const int N = fan[l], group = N <= 16 ? 32 / N : 1;
+            rounds += items * (l ? child.above[N] : g->roots.above[N]) / (group * (T / 32));
+            items *= l ? child.fill[N] : (float)N;
+        }
+        const int64_t room_chunks = (int64_t)g->sm_count * (1024 / T);
+        if (rounds * (double)((t->n_chunks + room_chunks - 1) / room_chunks) > TREE_CHUNK_ROUNDS) return false;
+    }
     for (int l = 0; l <= D; ++l) t->qoff[l] = off[l] * (uint32_t)C;
     t->wmax = wmax * (uint32_t)C;
     *threads = T;
@@ -588,7 +634,7 @@ int run_tree(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int fan[], 
     a.D = p->depth;
     for (int l = 0; l < p->depth; ++l) a.fan[l] = (uint8_t)fan[l];
     t.seeds = seeds;
-    t.n_samples = p->n_samples;
+    t.n_roots = p->n_samples * p->frontier_size;
     t.F = p->frontier_size;
     t.base = (int)p->sample_base;
     const DevGraph dg = dev_view(g, p->schedule, BIAS);
@@ -1395,6 +1441,15 @@ extern "C" int csaw_graph_create(const void *rowptr, int rowptr_is_64, const int
             if (!(weights[e] >= 0.f) || std::isinf(weights[e]))
                 return fail(CSAW_ERR_INVALID, "weights must be finite and >= 0");
     auto *g = new csaw_graph_s();
+    for (int64_t i = 0; n_edges > 0 && i < DEGREE_SAMPLE; ++i) {
+        const int64_t v = (int64_t)((double)i * (double)n_vertices / DEGREE_SAMPLE), dv = rp(v + 1) - rp(v);
+        if (dv > 0) g->roots.add(dv, 1.0);
+        const int64_t u = col[(int64_t)((double)i * (double)n_edges / DEGREE_SAMPLE)], du = rp(u + 1) - rp(u);
+        g->children[0].add(du, 1.0);
+        g->children[1].add(du, (double)du);
+    }
+    g->roots.finish();
+    for (DegreeShare &c : g->children) c.finish();
     cudaGetDevice(&g->device);
     cudaDeviceGetAttribute(&g->sm_count, cudaDevAttrMultiProcessorCount, g->device);
     int l2 = 0;

@@ -1,8 +1,9 @@
 // kernels_tree.cuh -- whole sample trees in one launch (sm_100a).
 //
-// Samples are independent, so a neighbor job needs no level-wide order: a CTA
-// takes a chunk of consecutive samples and runs all of their levels, the
-// frontier queue in shared memory, with CTA barriers between levels.  The
+// The trees of different seeds are independent (without dedup), so a neighbor
+// job needs no level-wide order: a CTA takes a chunk of consecutive roots, the
+// samples' seeds, and runs all levels of their trees, the frontier queue in
+// shared memory, with CTA barriers between levels.  The
 // per-level passes (kernels_fast.cuh) cost 6-8 launches a level, each several
 // microseconds however few items it finds; a small or middle-sized job is
 // nothing but those launches.  Here it is one launch whose length is the
@@ -10,9 +11,13 @@
 //   scan    every item's edge count, items that need draws (d > N) listed; the
 //           chunk's output range is reserved by one atomic, whose round trip
 //           the first selections hide (edges are written past a second barrier)
-//   draw    listed items 32 / N a warp (cached, N <= 16, d >= 3N: group_select)
-//           or a warp each, taken from shared counters so that warps that
-//           meet long items take fewer
+//   draw    listed items 32 / N a warp (group_select) where N <= 16 and few
+//           first phases fail -- d >= 3N over a cached prefix, d >= 2N unbiased,
+//           any d for N <= 4 -- or a warp each, taken from shared counters so
+//           that warps that meet long items take fewer.  (A warp each for
+//           unbiased and for short rows of few slots: 200,000 seeds [2] on the
+//           power-law graph, edge weights, 119 us, 80 so; 1024 unbiased seeds
+//           [15,10,5] on R-MAT 22 119 and 69.)
 //   expand  take-all items by flattened batches, as the take-all pass does
 //   retry   cached hubs whose first phase failed, the whole CTA on each
 // A selected edge's child goes straight to the next level's queue slot (the
@@ -41,7 +46,7 @@ constexpr int TREE_MAX_ITEMS = 4096;   // queue entries of a chunk, all levels (
 struct TreeArgs {
     LevelArgs lv;                          // outputs, keys, counters, scratch, fan, D (queue fields unused)
     const int32_t *seeds;
-    int n_samples, F, base, per_chunk, n_chunks;
+    int n_roots, F, base, per_chunk, n_chunks;   // roots: the samples' seeds, F a sample
     uint32_t qoff[TREE_MAX_LEVELS + 1];    // first queue entry of level l; [D] the chunk's total
     uint32_t wmax;                         // entries of the widest level
     CounterOut done;
@@ -73,17 +78,18 @@ __host__ __device__ __forceinline__ TreeSmem tree_smem(int nw, uint32_t qtot, ui
     m.list = at;
     at += (wmax * 2u + 3u) & ~3u;
     m.glist = at;
-    at += biased ? (wmax * 2u + 3u) & ~3u : 0u;
+    at += (wmax * 2u + 3u) & ~3u;
     m.retry = at;
     at += biased ? (wmax * 2u + 3u) & ~3u : 0u;
     m.bytes = at;
     return m;
 }
 
-// First phase of 32 / N items of a cached prefix, slot sl of the lane's item
-// on lane first + sl (lanes of gmask), as the group pass runs it.  cand: the
-// lane's index.  Returns -1, or the slot of the lane's item whose draws ran
-// out (the slots before it are accepted).
+// First phase of 32 / N items, slot sl of the lane's item on lane first + sl
+// (lanes of gmask), as the group pass runs it; biased ones over a cached
+// prefix.  cand: the lane's index.  Returns -1, or the slot of the lane's item
+// whose draws ran out (the slots before it are accepted).
+template <bool BIASED>
 __device__ __forceinline__ int group_select(const DevGraph &g, int64_t beg, int d, int N, const DrawCtx &dc, bool act,
                                             unsigned gmask, int first, int sl, int lane, int &cand) {
     const unsigned below = gmask & ((1u << lane) - 1u);
@@ -91,15 +97,19 @@ __device__ __forceinline__ int group_select(const DevGraph &g, int64_t beg, int 
     uint4 blk = make_uint4(0u, 0u, 0u, 0u);
     int used = 0, fail = -1, c = -2 - lane;
     if (act) {
-        T = __ldg(g.cdf + beg + d - 1);
+        if (BIASED) T = __ldg(g.cdf + beg + d - 1);
         blk = philox(make_uint4(dc.p, dc.s, (TAG_SAMPLE << 24) | dc.l, (uint32_t)sl << 16), dc.k0, dc.k1);
     }
     bool draw = act;
 #pragma unroll 1
     for (;;) {
         if (draw) {
-            c = cdf_find(g, beg, d, word_of(blk, used), T);
-            if (!(T > 0.f)) c = sl;
+            if (BIASED) {
+                c = cdf_find(g, beg, d, word_of(blk, used), T);
+                if (!(T > 0.f)) c = sl;
+            } else {
+                c = (int)mulhi(word_of(blk, used), (uint32_t)d);
+            }
             ++used;
             cand = c;
         }
@@ -154,18 +164,18 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
 
     for (int chunk = blockIdx.x; chunk < t.n_chunks; chunk += gridDim.x) {
         const int c0 = chunk * t.per_chunk;
-        const int ns = t.n_samples - c0 < t.per_chunk ? t.n_samples - c0 : t.per_chunk;
-        uint32_t n = (uint32_t)(ns * t.F);
+        uint32_t n = (uint32_t)(t.n_roots - c0 < t.per_chunk ? t.n_roots - c0 : t.per_chunk);
         for (uint32_t i = tid; i < n; i += T) {
-            int32_t v = __ldg(t.seeds + (int64_t)c0 * t.F + i);
+            const uint32_t root = (uint32_t)c0 + i;
+            int32_t v = __ldg(t.seeds + root);
             if (v < 0 || v >= g.v.n_vertices) {
                 atomicOr(a.err, ERR_SEED_RANGE);
                 v = 0;
             }
             const int64_t b = row_begin<I>(g, v);
             qv[i] = v;
-            qs[i] = t.base + c0 + (int32_t)(i / (uint32_t)t.F);
-            qp[i] = i % (uint32_t)t.F;
+            qs[i] = t.base + (int32_t)(root / (uint32_t)t.F);
+            qp[i] = root % (uint32_t)t.F;
             qb[i] = (I)b;
             qd[i] = (int32_t)(row_begin<I>(g, v + 1) - b);
         }
@@ -176,7 +186,8 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
             const uint32_t Q = t.qoff[l], Qn = t.qoff[l + 1];
             const unsigned long long per_edge = 4ull + 4ull * nout + (push ? 12ull + 2 * (sizeof(I) + 4) : 0ull);
             // ---- scan: output offsets and the lists of items that need draws
-            const bool grouped = BIASED && N <= 16;
+            const bool grouped = N <= 16;
+            const int dgroup = N <= 4 ? N + 1 : (BIASED ? CSAW_PAIR_MIN_RATIO * N : 2 * N);
             uint32_t total = 0;
             for (uint32_t b0 = 0; b0 < n; b0 += T) {
                 const uint32_t i = b0 + tid;
@@ -187,7 +198,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                     const int incl = warp_incl_scan(k, lane);
                     excl = (uint32_t)(incl - k);
                     if (lane == 31) s_w[warp] = (uint32_t)incl;
-                    const bool drawn = d > N, grp = drawn && grouped && d >= CSAW_PAIR_MIN_RATIO * N;
+                    const bool drawn = d > N, grp = drawn && grouped && d >= dgroup;
                     const unsigned gm = __ballot_sync(FULL, grp), wm = __ballot_sync(FULL, drawn && !grp);
                     uint32_t pg = 0, pw = 0;
                     if (n <= 32) {
@@ -304,10 +315,10 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                         ig = act ? glist[x + gi] : 0u;
                         const int d = qd[Q + ig];
                         const DrawCtx dc{a.k0, a.k1, qp[Q + ig], (uint32_t)qs[Q + ig], (uint32_t)l};
-                        fg = group_select(g, (int64_t)qb[Q + ig], d, N, dc, act, gmask, first, sl, lane, cg);
+                        fg = group_select<BIASED>(g, (int64_t)qb[Q + ig], d, N, dc, act, gmask, first, sl, lane, cg);
                         const bool failed = act && fg >= 0;
-                        if (failed && sl == 0 && d > WF) retry[atomicAdd(&s_nretry, 1u)] = (uint16_t)ig;
-                        pend = __ballot_sync(FULL, failed && sl == 0 && d <= WF);
+                        if (BIASED && failed && sl == 0 && d > WF) retry[atomicAdd(&s_nretry, 1u)] = (uint16_t)ig;
+                        pend = __ballot_sync(FULL, failed && sl == 0 && (!BIASED || d <= WF));
                         act = act && !failed;
                         i = ig;
                         j = sl;

@@ -90,6 +90,56 @@ def test_hub_resume_by_both_routes(csaw, concentrated, rowptr64, bias, fan):
     G.close()
 
 
+def regular(V, d, seed):
+    """V vertices of d distinct neighbors each, uniform weights."""
+    from csaw import graphgen
+    rng = np.random.default_rng(seed)
+    step = rng.permutation(np.arange(1, V))[:d]
+    col = (np.arange(V)[:, None] + np.sort(step)[None, :]) % V
+    col.sort(axis=1)
+    return graphgen.CSR(np.arange(V + 1, dtype=np.int64) * d, col.reshape(-1).astype(np.int32),
+                        (rng.random(V * d) + 1e-3).astype(np.float32), name="regular")
+
+
+@pytest.mark.parametrize("bias,schedule", [(0, 0), (0, 1), (1, 1), (2, 1)])
+def test_wide_trees_of_few_roots_use_the_whole_gpu(csaw, bias, schedule):
+    """The default rule: a tree whose levels would keep one SM's warps waiting
+    goes by the per-level launches; the same fan-outs on short rows (taken
+    whole), the same items from more roots, and narrow levels go in one."""
+    long_rows, short_rows = regular(3000, 200, 1), regular(3000, 3, 2)
+    for g, n, F, fan, tree in ((long_rows, 4, 1, [32, 32, 32], 0), (long_rows, 1, 4, [31, 32, 32], 0),
+                               (short_rows, 4, 1, [32, 32, 32], 1), (long_rows, 64, 1, [25, 10], 1),
+                               (long_rows, 33, 32, [32], 1), (long_rows, 1, 600, [2, 2], 1)):
+        seeds = oracle.make_seeds(g.rowptr, n * F, 3)
+        G = csaw.Graph(g)
+        p = csaw.make_params(0, bias, n, F, fan[0], len(fan), fan, 0xD0, schedule=schedule)
+        got, kinds = run(G, p, seeds)
+        G.close()
+        assert kinds["tree"]["launches"] == tree, (g.name, g.rowptr[1], n, F, fan)
+        ref = expected(g, seeds, bias, n, F, fan, 0xD0)
+        assert got.shape == ref.shape and np.array_equal(got, ref), (n, F, fan)
+
+
+@pytest.mark.parametrize("bias,schedule", [(0, 0), (0, 1), (1, 1), (2, 1)])
+@pytest.mark.parametrize("d", [3, 4, 5, 9, 13, 17, 24, 31, 33])
+def test_grouped_draws_of_short_rows(csaw, d, bias, schedule):
+    """Rows around N, 2N and 3N edges, where grouped items' first phases fail
+    now and then or always, for one slot to sixteen."""
+    from csaw import _lib
+    g = regular(800, d, 40 + d)
+    G = csaw.Graph(g)
+    G.set_option(_lib.OPT_TREE, 2)
+    for k, fan in enumerate(([1, 3], [2, 4], [4, 2], [8, 2], [12, 1], [16, 2])):
+        n, F = 90, 3
+        seeds = oracle.make_seeds(g.rowptr, n * F, 7 + k)
+        p = csaw.make_params(0, bias, n, F, fan[0], 2, fan, 0xE0 + k, schedule=schedule)
+        got, kinds = run(G, p, seeds)
+        ref = expected(g, seeds, bias, n, F, fan, 0xE0 + k)
+        assert kinds["tree"]["launches"] == 1
+        assert got.shape == ref.shape and np.array_equal(got, ref), fan
+    G.close()
+
+
 def test_tree_option_range(csaw, powerlaw_small):
     from csaw import _lib
     G = csaw.Graph(powerlaw_small)
