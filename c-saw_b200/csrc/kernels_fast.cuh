@@ -1118,11 +1118,9 @@ k_walk_fast(DevGraph g, WalkArgs a) {
                         n = d - lo < step ? d - lo : step;
                     }
                 } else {
-                    const int o2 = (int)(beg & 1023), last = o2 + d - 1;   // the row's ends, from its first group
-                    const int64_t b0 = beg - o2;
-                    const int ng = (last >> 10) + 1;
-                    const float *c2 = g.cdf2 + (b0 >> 10);
-                    int u = 0, m = ng;
+                    const RowSpan row = row_span(beg, d);
+                    const float *c2 = g.cdf2 + (row.b0 >> 10);
+                    int u = 0, m = (int)(row.last >> 10) + 1;
                     T = __ldg(cp + d - 1);
                     do {   // the last group's entry is never read: it is known to exceed the target
                         const int st = (m + 31) >> 5, q = u + (lane + 1) * st - 1;
@@ -1132,12 +1130,13 @@ k_walk_fast(DevGraph g, WalkArgs a) {
                         m = m - k * st < st ? m - k * st : st;
                         u += k * st;
                     } while (m > 1);
-                    const int ka = max(u << 5, o2 >> 5), kb = min((u << 5) + 31, last >> 5);   // its tiles
+                    const int ka = max(u << 5, (int)(row.o2 >> 5));   // its tiles
+                    const int kb = min((u << 5) + 31, (int)(row.last >> 5));
                     const int q = ka + lane;
-                    pv = q < kb ? __ldg(g.cdf1 + (b0 >> 5) + q) : 0.f;
+                    pv = q < kb ? __ldg(g.cdf1 + (row.b0 >> 5) + q) : 0.f;
                     const int k = ka + __ffs(__ballot_sync(FULL, q >= kb || pv > tt)) - 1;
-                    lo = max((k << 5) - o2, 0);
-                    n = min((k << 5) + 31, last) - o2 - lo + 1;
+                    lo = tile_at(row, k) + tile_lo(row, k);
+                    n = tile_hi(row, k) - tile_lo(row, k);
                 }
                 const bool mine = lane < n;
                 if (d > 32) {
