@@ -200,6 +200,8 @@ struct csaw_graph_s {
     int retry_smem = 0;           // CSAW_OPT_RETRY_SMEM (bytes)
     bool persistent = false;      // CSAW_OPT_PERSISTENT
     int thread_sel = 1;           // CSAW_OPT_THREAD_SELECT: 0 off, 1 degree rule, 2 every d <= 32 item
+    uint32_t tuned = 0;           // options (bit: number) whose value the autotuner chose, not the caller
+    int64_t shaped_jobs = 0;      // neighbor jobs run so far whose launches the tuned options shape
     DegreeShare roots, children[2];   // of seeds drawn uniformly; of neighbors (and weighted by their degree)
     int tree = 1;                 // CSAW_OPT_TREE: 0 never, 1 by size, 2 wherever a sample fits
     uint32_t class_mask = 0x7f;   // classes the trained model picks (bit c)
@@ -543,6 +545,16 @@ constexpr int64_t TREE_JOB_ITEMS = 1 << 18;
 constexpr double TREE_CHUNK_ROUNDS = 20;
 constexpr int64_t DEGREE_SAMPLE = 1 << 14;   // vertices and edges a graph's DegreeShare is made of
 
+// A launch-shape option set by the caller keeps the launches that it shapes.
+// A shape that the autotuner picked for its batch does not: it stays in the
+// graph for every later job, also the small ones that one launch runs in half
+// the time (64 seeds [25,10] on R-MAT 22 57 us, by the per-level launches 112).
+bool shape_by_caller(const csaw_graph_s *g) {
+    auto caller = [&](int opt) { return !((g->tuned >> opt) & 1u); };
+    return (g->grid_pct != 100 && caller(CSAW_OPT_GRID_PCT)) || (!g->pair && caller(CSAW_OPT_PAIR)) ||
+           (g->persistent && caller(CSAW_OPT_PERSISTENT)) || g->thread_sel == 2;
+}
+
 template <typename I, int BIAS>
 bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], TreeArgs *t, int *threads) {
     constexpr bool BIASED = BIAS != CSAW_BIAS_UNBIASED;
@@ -551,8 +563,7 @@ bool tree_shape(const csaw_graph_s *g, const csaw_params *p, const int fan[], Tr
     if (BIASED && (plain || g->cdf_off)) return false;
     if ((p->flags & CSAW_PARAM_DEDUP) && D > 1) return false;
     if (D > TREE_MAX_LEVELS || g->E == 0 || g->tree == 0) return false;
-    // launch-shape options keep the launches they shape
-    if (g->tree == 1 && !plain && (g->persistent || g->grid_pct != 100 || !g->pair || g->thread_sel == 2)) return false;
+    if (g->tree == 1 && !plain && shape_by_caller(g)) return false;
     if (p->schedule == CSAW_SCHED_LEARNED && BIASED) {   // only where the degree rule routes
         const bool model = g->trained && (g->class_mask & 0x7cu) && !g->mlp_lost && !(g->trial && g->trial_arm == 0);
         if (g->recording || model) return false;
@@ -670,6 +681,7 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
     if (B < 1) B = 1;
     const int64_t qcap = (int64_t)(B * per_sample) + 32;
     const bool plain = p->schedule == CSAW_SCHED_PLAIN;
+    if (!plain) ++g->shaped_jobs;
     // per-sample dedup: a (sample, vertex) table for every item one chunk can
     // queue (all levels that push), at most half full
     const bool dedup = (p->flags & CSAW_PARAM_DEDUP) != 0 && D > 1;
@@ -1980,10 +1992,12 @@ extern "C" int csaw_graph_set_option(csaw_graph g, int option, int64_t value) {
         case CSAW_OPT_GRID_PCT:
             if (value < 25 || value > 400) return fail(CSAW_ERR_INVALID, "grid percent must be in [25, 400]");
             g->grid_pct = (int)value;
+            g->tuned &= ~(1u << CSAW_OPT_GRID_PCT);
             ++g_alloc_epoch;   // launch shapes are baked into cached graphs
             return 0;
         case CSAW_OPT_PAIR:
             g->pair = value != 0;
+            g->tuned &= ~(1u << CSAW_OPT_PAIR);
             ++g_alloc_epoch;
             return 0;
         case CSAW_OPT_HOST_PARTS:
@@ -2006,6 +2020,7 @@ extern "C" int csaw_graph_set_option(csaw_graph g, int option, int64_t value) {
             return 0;
         case CSAW_OPT_PERSISTENT:
             g->persistent = value != 0;
+            g->tuned &= ~(1u << CSAW_OPT_PERSISTENT);
             ++g_alloc_epoch;   // launch structure is baked into cached graphs
             return 0;
         case CSAW_OPT_RETRY_SMEM:
@@ -2025,10 +2040,15 @@ extern "C" int csaw_graph_autotune(csaw_graph g, csaw_job *jobs, int n_jobs, voi
     const int pcts[3] = {100, 50, 200};
     const int old_pct = g->grid_pct;
     const bool old_pair = g->pair, old_graphs = g->use_graphs, old_persist = g->persistent;
-    g->use_graphs = false;   // each candidate timed launch by launch
+    const uint32_t old_tuned = g->tuned;
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
+    g->use_graphs = false;   // each candidate timed launch by launch
+    // candidates shape the launches that have a shape: jobs whose sample trees
+    // run in one launch do so under each of them, as they will afterwards
+    g->tuned = (1u << CSAW_OPT_GRID_PCT) | (1u << CSAW_OPT_PAIR) | (1u << CSAW_OPT_PERSISTENT);
+    const int64_t shaped0 = g->shaped_jobs;
     double best = 1e300, dflt = 0.0;
     int best_pct = old_pct, n = 0;
     bool best_pair = old_pair, best_persist = old_persist;
@@ -2051,7 +2071,7 @@ extern "C" int csaw_graph_autotune(csaw_graph g, csaw_job *jobs, int n_jobs, voi
         cudaEventElapsedTime(&ms, e0, e1);
         ++n;
         if (cand == 0) dflt = ms;
-        if (ms < best) {
+        if (ms < best && (cand == 0 || g->shaped_jobs != shaped0)) {   // nothing shaped: the default
             best = ms;
             best_pct = g->grid_pct;
             best_pair = pair != 0;
@@ -2065,6 +2085,7 @@ extern "C" int csaw_graph_autotune(csaw_graph g, csaw_job *jobs, int n_jobs, voi
         g->grid_pct = old_pct;
         g->pair = old_pair;
         g->persistent = old_persist;
+        g->tuned = old_tuned;
         return rc;
     }
     g->grid_pct = best_pct;

@@ -259,8 +259,9 @@ enum {
     /* Whole sample trees in one launch (neighbor jobs without dedup of up to
      * 8 hops, unbiased or with the degree rule over a cached prefix, the
      * plain schedule's unbiased jobs among them).  1 (default): small and
-     * middle jobs, by size, unless one of the launch-shape options above is
-     * set; 0: never, a launch or more per level; 2: every job whose samples
+     * middle jobs, by size, unless the caller has set one of the launch-shape
+     * options above (a shape that csaw_graph_autotune picked leaves them as
+     * they are); 0: never, a launch or more per level; 2: every job whose samples
      * fit one CTA's shared memory (4096 frontier items a sample).  Never
      * changes the output. */
     CSAW_OPT_TREE = 10
@@ -273,7 +274,10 @@ int csaw_graph_set_option(csaw_graph g, int option, int64_t value);
  * each candidate
  * (per-level launches with grid 50/100/200 % x pairing on/off, and the
  * persistent job kernel with pairing), device-timed, after one untimed run
- * each, and keeps the fastest in the graph's options.  The jobs' outputs are
+ * each, and keeps the fastest in the graph's options.  Jobs whose sample trees
+ * run in one launch (CSAW_OPT_TREE) have no such shape and keep that route,
+ * while the batch is timed and afterwards; a batch of them alone keeps the
+ * default shape.  The jobs' outputs are
  * overwritten by the runs (identical under every candidate).
  */
 typedef struct {
