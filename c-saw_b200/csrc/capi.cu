@@ -8,6 +8,7 @@
 // stream.  Errors are returned as status codes with a per-thread message.
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -618,8 +619,10 @@ int run_tree(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int fan[], 
     if (!plain) TRY(ensure_nbr(g, st));
     if (BIASED) TRY((ensure_cdf<I, BIAS>(g, st)));
     const TreeSmem m = tree_smem(threads / 32, t.qoff[p->depth], t.wmax, sizeof(I), BIASED);
-    static uint64_t attr_set = 0;   // per instantiation: bit = device
-    if (g->device < 64 && !((attr_set >> g->device) & 1u)) {
+    // per instantiation: bit = device; several threads may run jobs (of graphs
+    // of their own), and each may be the first
+    static std::atomic<uint64_t> attr_set{0};
+    if (g->device < 64 && !((attr_set.load() >> g->device) & 1u)) {
         CK(cudaFuncSetAttribute(k_tree<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 << 10));
         attr_set |= 1ull << g->device;
     }
@@ -781,8 +784,8 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
     const DevGraph dg = dev_view(g, p->schedule, BIAS);
     const uint64_t seed = p->seed;
     if (!plain && cached && g->maxdeg > WF) {
-        static uint64_t smem_set = 0;   // per instantiation: bit = device
-        if (g->device < 64 && !((smem_set >> g->device) & 1u)) {
+        static std::atomic<uint64_t> smem_set{0};   // per instantiation: bit = device
+        if (g->device < 64 && !((smem_set.load() >> g->device) & 1u)) {
             CK(cudaFuncSetAttribute(k_expand_heavy<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     RETRY_SMEM_MAX));
             smem_set |= 1ull << g->device;

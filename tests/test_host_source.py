@@ -1,0 +1,23 @@
+"""CPU checks of the host sources for state that several threads share: a graph
+serves one thread at a time, but threads with graphs of their own (a server's
+worker among them) run the same host code together."""
+import glob
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SOURCES = sorted(glob.glob(os.path.join(ROOT, "c-saw_b200", "csrc", "*.cu*")))
+
+SAFE = r"(?:const\b|constexpr\b|thread_local\b|std::atomic\b|std::mutex\b|std::once_flag\b|__device__\b|__global__\b|inline\b)"
+
+
+def test_function_statics_are_safe_between_threads():
+    """A variable of static duration inside a function is constant, atomic or
+    the thread's own."""
+    assert SOURCES
+    found = []
+    for path in SOURCES:
+        for n, line in enumerate(open(path).read().splitlines(), 1):
+            if re.match(r"\s+static\s+(?!" + SAFE + r")[^(]*[={;]", line):
+                found.append((os.path.basename(path), n, line.strip()))
+    assert not found, found
