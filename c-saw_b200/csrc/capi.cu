@@ -82,8 +82,10 @@ struct DevBuf {
 };
 
 // Bumped whenever a device buffer is (re)allocated: cached CUDA graphs that
-// captured older addresses are dropped.
-uint64_t g_alloc_epoch = 1;
+// captured older addresses are dropped.  One count for all graphs and their
+// threads: a plain one could lose an increment or take a later value back, and
+// a graph that had dropped its captures would take them for valid again.
+std::atomic<uint64_t> g_alloc_epoch{1};
 
 // Grows b to at least `bytes`.  With a stream that is not capturing, the old
 // buffer is released and the new one taken stream-ordered (after the work

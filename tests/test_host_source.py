@@ -21,3 +21,16 @@ def test_function_statics_are_safe_between_threads():
             if re.match(r"\s+static\s+(?!" + SAFE + r")[^(]*[={;]", line):
                 found.append((os.path.basename(path), n, line.strip()))
     assert not found, found
+
+
+def test_globals_are_safe_between_threads():
+    """So is a variable at namespace scope (named g_...)."""
+    found, seen = [], 0
+    for path in SOURCES:
+        for n, line in enumerate(open(path).read().splitlines(), 1):
+            m = re.match(r"(?:static\s+)?(?P<type>[A-Za-z_][\w:<>, ]*?)\s+g_\w+\s*(?:[={;\[])", line)
+            if m:
+                seen += 1
+                if not re.match(SAFE, m["type"]):
+                    found.append((os.path.basename(path), n, line.strip()))
+    assert seen and not found, found
