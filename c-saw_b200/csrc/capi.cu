@@ -1114,6 +1114,9 @@ int run_walk_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
     return 0;
 }
 
+constexpr int MDRW_SMEM_MAX = 96 * 1024;   // dynamic shared memory of a k_mdrw block, at most
+static_assert(12 * MDRW_MAX_F <= MDRW_SMEM_MAX, "one warp's frontier fits");
+
 template <typename I, int BIAS>
 int run_mdrw_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *seeds, const OutArgs &o,
                cudaStream_t st) {
@@ -1145,11 +1148,13 @@ int run_mdrw_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int32_t *
         return 0;
     }
     const size_t per_warp = (size_t)12 * a.F;
-    int wpb = (int)(96 * 1024 / per_warp);
+    int wpb = (int)(MDRW_SMEM_MAX / per_warp);
     if (wpb > WALK_THREADS / 32) wpb = WALK_THREADS / 32;
     if (wpb < 1) wpb = 1;
     const size_t dyn = per_warp * wpb;
-    CK(cudaFuncSetAttribute(k_mdrw<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    // the limit is the kernel's, not this call's: a value of this F could refuse
+    // the launch that another thread is about to make with a larger one
+    CK(cudaFuncSetAttribute(k_mdrw<I, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, MDRW_SMEM_MAX));
     int gmax = grid_for(k_mdrw<I, BIAS>, 32 * wpb, dyn, g->sm_count);
     int grid = (p->n_samples + wpb - 1) / wpb;
     if (grid > gmax) grid = gmax;

@@ -34,3 +34,14 @@ def test_globals_are_safe_between_threads():
                 if not re.match(SAFE, m["type"]):
                     found.append((os.path.basename(path), n, line.strip()))
     assert seen and not found, found
+
+
+def test_shared_memory_limits_do_not_depend_on_the_call():
+    """A kernel's limit of dynamic shared memory holds for the whole process,
+    so it is set to one constant and never to what one call needs."""
+    seen = 0
+    for path in SOURCES:
+        for value in re.findall(r"MaxDynamicSharedMemorySize,\s*([^;]*?)\)\)?;", open(path).read()):
+            seen += 1
+            assert re.fullmatch(r"[A-Z][A-Z0-9_]*|\d+( << \d+)?", value.strip()), (os.path.basename(path), value)
+    assert seen
