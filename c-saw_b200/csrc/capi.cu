@@ -133,9 +133,19 @@ constexpr size_t MAX_WARM = 1024;                   // batch keys remembered for
 // Job 0 serves csaw_sample; csaw_sample_batch runs job i on context i, each
 // on its own stream, so independent jobs overlap on the device.
 struct JobCtx {
-    DevBuf q[2][5], heavy, sel, hlist, hscratch, wscratch, seeds_in, out_dev, cta[4], retry, stab, hubsel, pairsel, dedup,
+    DevBuf q[2][5], heavy, sel, hscratch, wscratch, seeds_in, out_dev, cta[4], retry, stab, hubsel, pairsel, dedup,
         pctr,   // per-level counters and barrier words of a persistent job
         tsel;   // thread-per-item list
+    // all of them: what a job counts as its workspace, and what its end frees
+    template <typename F>
+    void each_buffer(F f) const {
+        for (auto &qq : q)
+            for (auto &b : qq) f(b);
+        for (auto &b : cta) f(b);
+        for (const DevBuf *b : {&heavy, &sel, &hscratch, &wscratch, &seeds_in, &out_dev, &retry, &stab, &hubsel,
+                                &pairsel, &dedup, &pctr, &tsel})
+            f(*b);
+    }
     Counters *ctr = nullptr, *hctr = nullptr;
     bool ctr_zero = false;           // ctr is zero once the work queued so far is done
     bool self_count = false;         // a job's only kernel may read its counters back itself ...
@@ -1212,11 +1222,7 @@ void free_job(JobCtx *c) {
     if (!c) return;
     if (c->copy) cudaStreamDestroy(c->copy);
     if (c->posts) cudaFreeHost(c->posts);
-    for (auto &qq : c->q)
-        for (auto &b : qq) cudaFree(b.p);
-    for (DevBuf *b : {&c->heavy, &c->sel, &c->hlist, &c->hscratch, &c->wscratch, &c->seeds_in, &c->out_dev, &c->cta[0],
-                      &c->cta[1], &c->cta[2], &c->cta[3], &c->retry, &c->stab, &c->hubsel, &c->pairsel, &c->dedup})
-        cudaFree(b->p);
+    c->each_buffer([](const DevBuf &b) { cudaFree(b.p); });
     cudaFree(c->ctr);
     if (c->hctr) cudaFreeHost(c->hctr);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -1231,11 +1237,7 @@ void free_job(JobCtx *c) {
 
 int64_t job_workspace(const JobCtx *c) {
     int64_t ws = 0;
-    for (auto &qq : c->q)
-        for (auto &b : qq) ws += (int64_t)b.n;
-    for (const DevBuf *b : {&c->heavy, &c->sel, &c->hlist, &c->hscratch, &c->wscratch, &c->seeds_in, &c->out_dev,
-                            &c->cta[0], &c->cta[1], &c->cta[2], &c->cta[3], &c->retry, &c->stab, &c->hubsel, &c->pairsel, &c->dedup})
-        ws += (int64_t)b->n;
+    c->each_buffer([&](const DevBuf &b) { ws += (int64_t)b.n; });
     return ws;
 }
 
