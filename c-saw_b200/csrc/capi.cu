@@ -923,7 +923,7 @@ int run_neighbor_t(csaw_graph_s *g, JobCtx *c, const csaw_params *p, const int f
                 a.n_refill = &pc[l].n_refill;
                 a.thread_list = nullptr;   // the thread pass's registers do not fit the persistent kernel
                 a.n_thread = &pc[l].n_thread;
-                a.refill_list = (SelEntry *)c->cta[1].p;   // the warp list is still being read beside the pair pass
+                a.refill_list = (SelEntry *)c->cta[1].p;   // the warp list is still being read beside the group pass
                 pa.lv[l] = a;
                 LevelArgs ar = a;
                 ar.sel_list = a.refill_list;
@@ -1343,8 +1343,6 @@ int finish_job(csaw_graph_s *g, JobCtx *c, int64_t cap, int64_t *n_out) {
     if (k.err & ERR_UPDATE_RANGE) return fail(CSAW_ERR_DEVICE, "Update() returned a vertex out of range");
     if (k.err & ERR_BARRIER)
         return fail(CSAW_ERR_DEVICE, "a grid barrier of the persistent job kernel expired (bounded wait)");
-    if (k.err & ERR_COPY_WAIT)
-        return fail(CSAW_ERR_DEVICE, "an asynchronous row copy did not complete within its bounded wait");
     if (k.err) return fail(CSAW_ERR_DEVICE, "kernel error flag " + std::to_string(k.err));
     if ((int64_t)k.out_count > cap)
         return fail(CSAW_ERR_CAPACITY, "output capacity " + std::to_string(cap) + " < " +

@@ -861,7 +861,7 @@ __device__ __forceinline__ void group_body(const DevGraph &g, const LevelArgs &a
     const uint32_t G = 32 / N;
     const uint32_t gi = (uint32_t)lane / (uint32_t)N;
     const int first = (int)gi * N, sl = lane - first;   // the item's first lane, the lane's slot
-    const unsigned gmask = gi < G ? (N == 32 ? FULL : ((1u << N) - 1u)) << first : 0u;
+    const unsigned gmask = gi < G ? ((1u << N) - 1u) << first : 0u;   // N <= 16
     const unsigned below = gmask & ((1u << lane) - 1u);
     const bool rec = a.sched && a.sched->mode == SCHED_RECORD;
     uint32_t my_items = 0, my_probes = 0;

@@ -225,7 +225,7 @@ k_expand_warp(DevGraph g0, LevelArgs a) {
                 sel = select_warp<I, BIAS, STREAM>(g, beg, d, N, dc, P, zb, zs, lane, WBUF,
                                                    STREAM && a.row_total ? __ldg(a.row_total + v) : -1.f);
                 if (sel == -2) {   // cached hub that needs a rebuild: the CTA path redoes it
-                    // (only with a prefix cache, which streaming graphs do not have)
+                    // (only with a prefix cache, resident or a streaming graph's)
                     my_items--;
                     if (lane == 0) {
                         uint32_t h = atomicAdd(a.n_heavy, 1u);
