@@ -995,9 +995,11 @@ def profile_kernels(args):
     (.6/.2/.15) scale 22, edge factor 16, int64 row offsets, Pareto(1.5)
     weights.  Runs, in order: the graph's prefix cache and neighbor records
     (first batched biased job), a batched F8 N10 D3 step with walks of 40
-    (take-all, warp-list, pair, retry, thread-per-walk passes), a batched
-    N 20 job (hub list), the plain schedule (warp expansion, CTA expansion,
-    warp walks), batched warp walks, MDRW, per-sample dedup, profile
+    (take-all, warp-list, group, retry, thread-per-walk passes), a batched
+    N 20 job (hub list), sample trees in one launch (1024 seeds [25, 10]),
+    the plain schedule (warp expansion, CTA expansion,
+    warp walks), batched warp walks, unbiased walks by column, MDRW with small
+    and large frontiers, per-sample dedup, profile
     recording and training of the learned scheduler, streaming through a
     512 MiB partition budget, and the allocation-free entry.  Prints the
     per-kind kernel statistics of each part."""
@@ -1028,11 +1030,13 @@ def profile_kernels(args):
     step = [job(0, 2, 8192, 8, 10, 3, seed=2), job(1, 2, 131072, 1, 1, 40, seed=3)]
     part("cache_build_and_first_step", lambda: G.sample_batch(step))
     part("batched_step", lambda: G.sample_batch(step))
-    part("batched_n20_hubs", lambda: G.sample_batch([job(0, 2, 2048, 4, 20, 2, seed=4)]))
+    part("batched_n20_hubs", lambda: G.sample_batch([job(0, 2, 4096, 4, 20, 2, seed=4)]))
+    part("trees", lambda: G.sample_batch([job(0, 2, 1024, 1, 25, 2, fan=[25, 10], seed=14)]))
     part("plain", lambda: G.sample_batch([job(0, 2, 256, 8, 10, 3, sched=csaw.SCHED_PLAIN, seed=5),
                                           job(1, 2, 2048, 1, 1, 40, sched=csaw.SCHED_PLAIN, seed=6)]))
     part("batched_warp_walks", lambda: G.sample_batch([job(1, 2, 4096, 1, 1, 40, seed=7)]))
-    part("mdrw", lambda: G.sample_batch([job(2, 1, 8192, 8, 1, 20, seed=8)]))
+    part("unbiased_walks", lambda: G.sample_batch([job(1, 0, 262144, 1, 1, 40, seed=15)]))
+    part("mdrw", lambda: G.sample_batch([job(2, 1, 8192, 8, 1, 20, seed=8), job(2, 1, 2048, 64, 1, 20, seed=16)]))
     part("dedup", lambda: G.sample_batch([job(0, 2, 4096, 4, 10, 3, dedup=True, seed=9)]))
     learn = [job(0, 2, 4096, 8, 10, 3, sched=csaw.SCHED_LEARNED, seed=10)]
     G.sched_record(100_000)

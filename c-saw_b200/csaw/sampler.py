@@ -299,7 +299,8 @@ class StreamGraph:
     def cache(self, bias):
         """Builds the prefix cache of `bias` (csaw_stream_graph_cache): later
         jobs with that bias stream each partition's prefix instead of its
-        weights and search it (the same edges)."""
+        weights and search it (the same edges).  Takes 0.13 bytes an edge and 4
+        a vertex of device memory beside slot_budget_bytes."""
         check(lib().csaw_stream_graph_cache(self.h, BIAS_NAMES.get(bias, bias)))
 
     def set_option(self, option, value):

@@ -51,7 +51,9 @@ enum {
 };
 
 enum {
-    CSAW_SCHED_PLAIN = 0,    /* one launch per level, degree-threshold rule */
+    CSAW_SCHED_PLAIN = 0,    /* one launch per level, degree-threshold rule;
+                                small and middle unbiased neighbor jobs run
+                                their sample trees in one launch */
     CSAW_SCHED_BATCHED = 1,  /* per-level passes by item class, CUDA-graph
                                 replayed; small and middle neighbor jobs run
                                 their sample trees in one launch; the
@@ -235,7 +237,8 @@ enum {
      * cached hub items may use to rebuild a row's prefix: rows whose
      * rebuild fits are done in shared memory, larger ones in global scratch.
      * More shared memory means fewer resident CTAs; never changes the
-     * output. */
+     * output.  No effect on jobs whose sample trees run in one launch
+     * (CSAW_OPT_TREE): their retries use global scratch. */
     CSAW_OPT_RETRY_SMEM = 6,
     /* 1: batched neighbor jobs run all their levels in one persistent
      * cooperative kernel (items pushed for the next level are consumed in
@@ -388,8 +391,11 @@ enum { CSAW_STREAM_OPT_READ_IN_PLACE = 1 };
 int csaw_stream_graph_set_option(csaw_stream_graph g, int option, int64_t value);
 /* Builds the per-vertex prefix cache of a bias kind (DEGREE, EDGE_WEIGHT or
  * HOOK) for a streaming graph: every row's canonical prefix in page-locked
- * host memory (4 E bytes) and its two index levels on the device (4.13 E/32
- * bytes); later jobs with that bias stream each partition's prefix in place
+ * host memory (4 E bytes) and, on the device and outside slot_budget_bytes,
+ * its two index levels (4.13 E/32 bytes) and every row's total (4 V bytes,
+ * which spare a draw one read over the link; if they cannot be allocated, it
+ * reads the total from the prefix): 34 + 67 MB at R-MAT scale 24, 1.1 + 2.1 GB
+ * at scale 29.  Later jobs with that bias stream each partition's prefix in place
  * of its weights and search it instead of recomputing a row's prefix per
  * expansion (raw weights, for the rare rebuild after repeated collisions,
  * are read from the page-locked host array).  The in-memory cache's
