@@ -836,9 +836,9 @@ k_select_thread(DevGraph g, LevelArgs a) {
 // consumed warp list), larger ones by the CTA pass.
 //
 // What bounds it: dependent sector gathers (entry, total and tile line, edge
-// line, column) and the instructions of the rounds, about equally: 47% issue
-// active, 3.8 TB/s of DRAM, 19 cycles between a warp's instructions, 11 of
-// them waiting for loads (level 2 at R-MAT scale 22).  An item costs 270 warp
+// line, column) and the instructions of the rounds, about equally: 55% issue
+// active, 3.9 TB/s of DRAM, 20 cycles between a warp's instructions, 11 of
+// them waiting for loads (level 2 at R-MAT scale 22).  An item costs 285 warp
 // instructions; two items a warp in halves of their own, their rows staged
 // in shared memory by the bulk copy engine, cost 550, as the halves diverged
 // in draws and refinements and paid the staging per item.  The gathers need
@@ -1252,7 +1252,8 @@ k_walk_fast(DevGraph g, WalkArgs a) {
 // writes them a step later, when the reservation has come back beside the
 // step's own loads.  (Staging 64 edges a warp and waiting for the atomic of
 // each flush took 531 us for 262,144 unbiased walks of 40 on R-MAT 22; this
-// takes 318, and 247 by columns: scattered 32-byte sectors, 40 G a second.)
+// takes 318, and 247 by columns, 4.8 TB/s of DRAM in 32- and 64-byte
+// accesses: 99 bytes read a step.)
 constexpr int WALK_KEEP = 8;
 
 template <typename I, int BIAS>

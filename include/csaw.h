@@ -367,7 +367,9 @@ typedef struct {
     int64_t bytes_h2d;         /* adjacency bytes copied */
     int64_t kernel_launches;
     int64_t host_pinned_in_place; /* bit 0: col, bit 1: weights registered */
-    int64_t items_read_in_place;  /* pending items served from host memory (CSAW_STREAM_OPT_READ_IN_PLACE) */
+    int64_t items_read_in_place;  /* items whose partition was in host memory when their round began
+                                     (CSAW_STREAM_OPT_READ_IN_PLACE); the hops a walk goes on with
+                                     in the same launch are not counted */
 } csaw_stream_info;
 int csaw_stream_graph_create(const void *rowptr, int rowptr_is_64, const int32_t *col,
                              const float *weights, int64_t n_vertices, int64_t n_edges,
