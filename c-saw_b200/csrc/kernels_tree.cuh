@@ -29,8 +29,8 @@
 // total and lines, neighbor record, and the launch itself; 64 seeds [25,10]
 // take 27 us, 12 of them before the first draw is written.  64 registers a
 // thread keep 1024 threads an SM resident, at the price of some spilled
-// values (128 registers: 66 us a call for 64 seeds against 69, but 93
-// against 79 for 1024).
+// values in the biased kernels (128 registers: 66 us a call for 64 seeds against
+// 69, but 93 against 79 for 1024).
 //
 // Selections are those of the other passes (the same device functions, draw
 // keys and canonical prefix), so the edges are the same.
@@ -159,8 +159,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
         s_items[tid] = 0u;
     }
     if (tid == 0) s_ndraw = s_ngroup = s_next = s_nextg = s_nretry = 0u;
-    unsigned long long my_bytes = 0;
-    uint32_t my_items = 0;
+    uint32_t my_bytes = 0, my_items = 0;   // a chunk's bytes are below 2^23 (TREE_MAX_ITEMS)
 
     for (int chunk = blockIdx.x; chunk < t.n_chunks; chunk += gridDim.x) {
         const int c0 = chunk * t.per_chunk;
@@ -184,9 +183,12 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
             const int N = a.fan[l];
             const bool push = l + 1 < a.D;
             const uint32_t Q = t.qoff[l], Qn = t.qoff[l + 1];
-            const unsigned long long per_edge = 4ull + 4ull * nout + (push ? 12ull + 2 * (sizeof(I) + 4) : 0ull);
+            const uint32_t per_edge = 4u + 4u * (uint32_t)nout + (push ? 12u + 2u * ((uint32_t)sizeof(I) + 4u) : 0u);
             // ---- scan: output offsets and the lists of items that need draws
-            const bool grouped = N <= 16;
+            // (unbiased items that are no more than the warps take one each: there
+            // are no rounds to share, and a failed first phase starts over.  1000
+            // seeds [2,2] on R-MAT 16: 42.2 us a call in groups, 40.7 so)
+            const bool grouped = N <= 16 && (BIASED || n > (uint32_t)nw);
             const int dgroup = N <= 4 ? N + 1 : (BIASED ? CSAW_PAIR_MIN_RATIO * N : 2 * N);
             uint32_t total = 0;
             for (uint32_t b0 = 0; b0 < n; b0 += T) {
@@ -218,7 +220,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                     if (i < n) {
                         if (n <= 32) qo[i] = excl;
                         my_items++;
-                        my_bytes += 12 + sizeof(I) + 4 + (!drawn ? per_edge * (unsigned)k : 0ull);
+                        my_bytes += 12u + (uint32_t)sizeof(I) + 4u + (!drawn ? per_edge * (uint32_t)k : 0u);
                     }
                 }
                 __syncthreads();
@@ -298,7 +300,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                 unsigned pend = 0u;      // failed rows of the warp's last group, by first lane
                 uint32_t ig = 0u;        // the lane's item, index and failing slot in it
                 int cg = -1, fg = -1;
-                bool groups = grouped;
+                bool groups = ngroup > 0u;
                 for (;;) {
                     bool act;
                     uint32_t i;
@@ -329,8 +331,10 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                             const int ld = __ffs(pend) - 1;
                             pend &= pend - 1;
                             i = __shfl_sync(FULL, ig, ld);
-                            j0 = __shfl_sync(FULL, fg, ld);
-                            sel = __shfl_sync(FULL, cg, (ld + lane) & 31);
+                            if (BIASED) {   // unbiased items start over
+                                j0 = __shfl_sync(FULL, fg, ld);
+                                sel = __shfl_sync(FULL, cg, (ld + lane) & 31);
+                            }
                         } else {
                             uint32_t x = 0;
                             if (lane == 0) x = atomicAdd(&s_next, 1u);
@@ -362,7 +366,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                         const int kind = BIASED && d > WF ? 2 : 1;
                         const unsigned long long search =
                             !BIASED ? 0ull : (d <= WF ? 4ull * d : (unsigned long long)N * 4ull * (32 - __clz(d)));
-                        atomicAdd(&s_bytes[kind], 16ull + search + (unsigned long long)N * per_edge);
+                        atomicAdd(&s_bytes[kind], 16ull + search + (uint32_t)N * per_edge);
                         atomicAdd(&s_items[kind], 1u);
                     }
                 }
@@ -406,7 +410,7 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
                                                                  sh, 0, -1, rebuild_bytes);
                     if (warp == 0) emit(lane < N, i, lane, sel);
                     if (tid == 0) {
-                        s_bytes[3] += 12 + 2 * sizeof(I) + rebuild_bytes + (unsigned long long)N * per_edge +
+                        s_bytes[3] += 12 + 2 * sizeof(I) + rebuild_bytes + (uint32_t)N * per_edge +
                                       (unsigned long long)N * 4ull * (32 - __clz(d));
                         s_items[3] += 1u;
                     }
@@ -417,14 +421,17 @@ k_tree(const __grid_constant__ DevGraph g, const __grid_constant__ TreeArgs t) {
             n = push ? total : 0u;
             __syncthreads();
         }
+        if (my_bytes >= 1u << 31) {
+            atomicAdd(&s_bytes[0], (unsigned long long)my_bytes);
+            my_bytes = 0u;
+        }
     }
+    unsigned long long warp_bytes = my_bytes;
 #pragma unroll
-    for (int off = 16; off; off >>= 1) {
-        my_bytes += __shfl_xor_sync(FULL, my_bytes, off);
-        my_items += __shfl_xor_sync(FULL, my_items, off);
-    }
+    for (int off = 16; off; off >>= 1) warp_bytes += __shfl_xor_sync(FULL, warp_bytes, off);
+    my_items = __reduce_add_sync(FULL, my_items);
     if (lane == 0 && my_items) {
-        atomicAdd(&s_bytes[0], my_bytes);
+        atomicAdd(&s_bytes[0], warp_bytes);
         atomicAdd(&s_items[0], my_items);
     }
     __syncthreads();

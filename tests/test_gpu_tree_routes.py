@@ -140,6 +140,25 @@ def test_grouped_draws_of_short_rows(csaw, d, bias, schedule):
     G.close()
 
 
+@pytest.mark.parametrize("schedule", [0, 1])
+@pytest.mark.parametrize("d", [20, 33, 200])
+def test_unbiased_levels_around_the_warps_of_a_chunk(csaw, d, schedule):
+    """Unbiased levels of one item less than the 16 warps of a chunk of few
+    roots, as many, and one more: a warp each, or in groups."""
+    from csaw import _lib
+    g = regular(800, d, 60 + d)
+    G = csaw.Graph(g)
+    G.set_option(_lib.OPT_TREE, 2)
+    for k, fan in enumerate(([15, 4], [16, 4], [17, 4], [1, 16, 2], [5, 3, 2])):
+        seeds = oracle.make_seeds(g.rowptr, 20, 9 + k)
+        p = csaw.make_params(0, 0, 20, 1, fan[0], len(fan), fan, 0xF0 + k, schedule=schedule)
+        got, kinds = run(G, p, seeds)
+        ref = expected(g, seeds, 0, 20, 1, fan, 0xF0 + k)
+        assert kinds["tree"]["launches"] == 1
+        assert got.shape == ref.shape and np.array_equal(got, ref), fan
+    G.close()
+
+
 def test_tree_option_range(csaw, powerlaw_small):
     from csaw import _lib
     G = csaw.Graph(powerlaw_small)
